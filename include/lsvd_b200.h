@@ -361,7 +361,7 @@ typedef struct lsvd_gemv_args {
   int64_t residual_row_stride;
   int32_t* status_word;          /* device int32 or NULL: LSVD_ERR_TIMEOUT if a pipeline wait of the   */
                                  /* TMA-fed form ran out; the output is then incomplete               */
-  int32_t form;                  /* 0: chosen by size (2 beyond 32 tokens on large matrices, else 3);    */
+  int32_t form;                  /* 0: tcgen05 kernel, every size;                                        */
                                  /* 1: persistent TMA-fed kernel with K split over warps, m <= 16 only   */
                                  /*    (LSVD_ERR_UNSUPPORTED beyond); 2: TMA-fed kernel whose warps      */
                                  /*    share the token rows (built for 17..64 tokens, valid for any m);   */
@@ -370,9 +370,10 @@ typedef struct lsvd_gemv_args {
   int64_t row_absmax_stride;     /* words between two tokens                                              */
   int32_t absmax_split;          /* 0: one word per token; else channels >= absmax_split (a multiple of  */
                                  /* 16) go to the token's second word                                     */
-  int32_t prefetch_weights;      /* register-fed form: every block asks for its weight rows (L2 prefetch) before */
-                                 /* it waits for the kernel launched before it on the stream; pays when the       */
-                                 /* call follows a short kernel (measured: 126 -> 120 us for the mixffn step)      */
+  int32_t prefetch_weights;      /* every block asks for its weights (form 0: the first stages of its ring, form 3: */
+                                 /* L2 prefetch) before it waits for the kernel launched before it on the stream.    */
+                                 /* Set it only behind one of this library's kernels: the weights must be complete   */
+                                 /* when that kernel starts.  Results do not depend on it.                           */
   float* out_f32;                /* optional device fp32 [m, n] (single product, forms 0 and 3): (acc * a_scale) * w_scale  */
                                  /* with no fp16 rounding -- the partial sum a row-parallel rank sends to the all-reduce  */
 } lsvd_gemv_args;

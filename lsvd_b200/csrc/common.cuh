@@ -35,10 +35,8 @@ cudaError_t ensure_dynamic_smem(const void* kernel, int bytes);
 // with programmatic stream serialisation: the next kernel's blocks may become resident while the previous
 // kernel drains, and wait in grid_dependency_sync() (first statement of every such kernel) until the previous
 // grid has completed and its writes are visible.  LSVD_CHAINED_LAUNCH=0 in the environment turns it off.
-// The attention kernels use it.  On the FFN side only the mixffn quantisers and the products that ask for a weight
-// prefetch do (LSVD_CHAIN_FFN=0 turns those off): for the other quantisers and products it measured faster at 1..32
-// tokens (FFN block 52.5 / 56.8 instead of 56.9 / 59.2 us at 1 / 16 tokens) but slower at 64 tokens (143 instead of
-// 117 us) and behind the attention kernels (167 instead of 153 us for attention + FFN).
+// The attention kernels, the quantisers and the products that ask for a weight prefetch use it (LSVD_CHAIN_FFN=0 turns
+// the products' prefetch off).
 bool chained_launch_enabled();
 bool ffn_chain_enabled();
 
@@ -81,6 +79,12 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 __device__ __forceinline__ void grid_dependency_sync() {
   grid_dependency_release();
   grid_dependency_wait();
+}
+// The order of the quantisers: the kernel behind them may ask for its WEIGHTS before it waits, so it must not start before
+// everything in front of the quantiser (which may have written those weights) has completed.
+__device__ __forceinline__ void grid_dependency_wait_release() {
+  grid_dependency_wait();
+  grid_dependency_release();
 }
 
 // Record the first error code seen by a kernel; later codes do not overwrite it.

@@ -25,14 +25,14 @@ namespace lsvd {
 __global__ void __launch_bounds__(256) act_quant_kernel(const __grid_constant__ ActQuantParams p) {
   extern __shared__ float row[];          // cols floats
   __shared__ float red[8];
-  grid_dependency_sync();
+  grid_dependency_wait_release();
   act_quant_row(p, blockIdx.x, row, red);
 }
 
 __global__ void __launch_bounds__(256) act_quant_rot4096_kernel(const __grid_constant__ ActQuantParams p) {
   __shared__ float row[4096 + 256];
   __shared__ float red[8];
-  grid_dependency_sync();
+  grid_dependency_wait_release();
   act_quant_rot4096_row(p, blockIdx.x, row, red);
 }
 
@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(256) act_quant_rot4096_kernel(const __grid_con
 // is added in another order (lane-wise, then across the warp).
 template <int NCH>
 __global__ void __launch_bounds__(256, (NCH <= 16 ? 2 : 1)) act_quant_rows_kernel(const __grid_constant__ ActQuantParams p) {
-  grid_dependency_sync();
+  grid_dependency_wait_release();
   const int lane = threadIdx.x & 31;
   const int r = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (r >= p.rows) return;
@@ -133,7 +133,7 @@ struct HeadsHadParams {
 template <int H>
 __global__ void __launch_bounds__(128) heads_hadamard_quant_kernel(const __grid_constant__ HeadsHadParams p) {
   __shared__ float red[8];
-  grid_dependency_sync();
+  grid_dependency_wait_release();
   const int r = blockIdx.x, D = p.head_dim;
   const __half* x = p.x + r * p.x_row_stride;
   const int c = 2 * threadIdx.x;                  // columns c, c + 1
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(128) heads_hadk_quant_kernel(const __grid_cons
   float* hk = reinterpret_cast<float*>(hh_smem);                       // [H][H]
   __half2* ys = reinterpret_cast<__half2*>(hk + p.heads * p.heads);    // [H][D / 2]
   __shared__ float red[8];
-  grid_dependency_sync();
+  grid_dependency_wait_release();
   const int r = blockIdx.x, D = p.head_dim, H = p.heads;
   for (int i = threadIdx.x; i < H * H; i += blockDim.x) hk[i] = __half2float(had_K[i]);
   const __half* x = p.x + r * p.x_row_stride;
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(256) hadamard_quant_kernel(const __grid_consta
   __half* Tt = reinterpret_cast<__half*>(smem_raw);          // [ntile_per * 8][ld]: my columns of the rotated blocks
   __half* xs = Tt + p.ntile_per * 8 * p.ld;                  // [cols]: the token's row, staged with wide loads
   __shared__ float red[8];
-  grid_dependency_sync();
+  grid_dependency_wait_release();
   __shared__ float my_max;
   const int crank = static_cast<int>(cluster_rank());
   const int r = blockIdx.x / p.cluster;
@@ -745,7 +745,7 @@ static int launch_gemv_nt(const GemvParams& p, bool dual, bool split, cudaStream
 namespace lsvd {
 __global__ void dequant_residual_kernel(const int32_t* acc, const float* a_scale, const float* w_scale, const __half* residual,
                                         int64_t res_stride, __half* out, int64_t out_stride, int m, int n) {
-  grid_dependency_sync();
+  grid_dependency_wait_release();
   const int64_t total = static_cast<int64_t>(m) * n;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int tok = static_cast<int>(i / n), ch = static_cast<int>(i - static_cast<int64_t>(tok) * n);
@@ -804,7 +804,7 @@ extern "C" int lsvd_act_quant(const lsvd_act_quant_args* a, void* stream) {
   if (rotate && a->cols == 4096 && p.vec8 && p.norm_weight == nullptr && p.fake == nullptr && aligned(a->q, 16) && (a->q_row_stride % 16) == 0 &&
       (p.x_rot == nullptr || aligned(p.x_rot, 16))) {
     LSVD_CUDA_TRY(launch_chained(act_quant_rot4096_kernel, dim3(a->rows), dim3(256), 0, static_cast<cudaStream_t>(stream), 1,
-                                 false, p));
+                                 true, p));
     return LSVD_OK;
   }
   // many rows of a width the warp-per-row kernel is built for (a prefill): no shared memory, no block barriers
@@ -822,13 +822,13 @@ extern "C" int lsvd_act_quant(const lsvd_act_quant_args* a, void* stream) {
       default: break;
     }
     if (kern != nullptr) {
-      LSVD_CUDA_TRY(launch_chained(kern, dim3((a->rows + 7) / 8), dim3(256), 0, static_cast<cudaStream_t>(stream), 1, false, p));
+      LSVD_CUDA_TRY(launch_chained(kern, dim3((a->rows + 7) / 8), dim3(256), 0, static_cast<cudaStream_t>(stream), 1, true, p));
       return LSVD_OK;
     }
   }
   const int smem = a->cols * 4;
   if (smem > 48 * 1024) LSVD_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(act_quant_kernel), smem));
-  LSVD_CUDA_TRY(launch_chained(act_quant_kernel, dim3(a->rows), dim3(256), smem, static_cast<cudaStream_t>(stream), 1, false, p));
+  LSVD_CUDA_TRY(launch_chained(act_quant_kernel, dim3(a->rows), dim3(256), smem, static_cast<cudaStream_t>(stream), 1, true, p));
   return LSVD_OK;
 }
 
@@ -864,7 +864,7 @@ extern "C" int lsvd_heads_hadamard_quant(const lsvd_heads_hadamard_quant_args* a
     return LSVD_OK;
   }
   if (kern == nullptr) return LSVD_ERR_UNSUPPORTED;       // not a power of two and no had_K given
-  LSVD_CUDA_TRY(launch_chained(kern, dim3(a->rows), dim3(128), 0, static_cast<cudaStream_t>(stream), 1, false, p));
+  LSVD_CUDA_TRY(launch_chained(kern, dim3(a->rows), dim3(128), 0, static_cast<cudaStream_t>(stream), 1, true, p));
   return LSVD_OK;
 }
 
@@ -984,13 +984,13 @@ extern "C" int lsvd_hadamard_quant(const lsvd_hadamard_quant_args* a, void* stre
     if (smem_rows > 48 * 1024)
       LSVD_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(hadamard_quant_rows_kernel), smem_rows));
     LSVD_CUDA_TRY(launch_chained(hadamard_quant_rows_kernel, dim3(static_cast<unsigned>(a->rows)), dim3(p.Kp * 2), smem_rows,
-                                 static_cast<cudaStream_t>(stream), 1, false, p));
+                                 static_cast<cudaStream_t>(stream), 1, true, p));
     return LSVD_OK;
   }
   void (*kern)(HadQuantParams) = p.ntile_per <= 2 ? hadamard_quant_kernel<2> : hadamard_quant_kernel<8>;
   if (smem > 48 * 1024) LSVD_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
   LSVD_CUDA_TRY(launch_chained(kern, dim3(static_cast<unsigned>(a->rows * p.cluster)), dim3(256), smem,
-                               static_cast<cudaStream_t>(stream), p.cluster, false, p));
+                               static_cast<cudaStream_t>(stream), p.cluster, true, p));
   return LSVD_OK;
 }
 
@@ -1030,14 +1030,10 @@ extern "C" int lsvd_w8a8_gemv(const lsvd_gemv_args* a, void* stream) {
   if (a->form == 1) return a->m <= 16 ? launch_gemv_streamed(p, dual, split, st) : LSVD_ERR_UNSUPPORTED;
   if (a->form == 2) return launch_gemv_wide(p, dual, split, st);
   if (a->form != 0 && a->form != 3) return LSVD_ERR_INVALID_ARG;
-  // more than 32 tokens: the form that shares the token rows between a block's warps (measured: 35.6 vs 48.9 us for the
-  // 45 MB gate/up pair at 64 tokens; no gain at 32 tokens).  Its blocks split K between their warps when the matrix
-  // has few channels, which is what a tensor-parallel rank's column slice looks like (a 9.8 MB latent projection slice
-  // took 38 us in the register-fed form, more than the whole 39 MB matrix in this one); short reductions stay
-  // register-fed.
-  const int64_t weight_bytes = static_cast<int64_t>(a->n) * a->k * (dual ? 2 : 1);
-  if (a->form == 0 && !fp32_form && a->out_f32 == nullptr && a->m > 32 && weight_bytes >= (4ll << 20) && a->k >= 2048)
-    return launch_gemv_wide(p, dual, split, st);
+  // Form 0 at every size: at 1 token the tcgen05 form and the register-fed one are level on the 4 MB product (the chain's
+  // other kernels bound it) and 45 MB take 15 instead of 17 us with their quantiser; from 17 tokens on it is 1.3 to 3
+  // times as fast (figures in gemv_tc.cu).
+  if (a->form == 0) return launch_gemv_tc(p, dual, split, st);
   if (a->m <= 8) return launch_gemv_nt<1>(p, dual, split, st);
   if (a->m <= 16) return launch_gemv_nt<2>(p, dual, split, st);
   if (a->m <= 32) return launch_gemv_nt<4>(p, dual, split, st);

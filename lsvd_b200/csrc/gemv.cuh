@@ -18,7 +18,7 @@ struct GemvParams {
   // optional per-token maximum of |fp32 value| over the output channels, kept as the bit pattern of a non-negative
   // float (ordered like an unsigned integer): slot 0 for channels below absmax_split, slot 1 from there on
   uint32_t* row_absmax; int64_t row_absmax_stride; int32_t absmax_split;
-  int32_t prefetch;          // pull the block's weight rows toward L2 before waiting for the previous kernel
+  int32_t prefetch;          // request weights before waiting for the previous kernel (launched programmatically)
   float* out_f32;            // optional [m, n]: (acc * a_scale) * w_scale before any fp16 rounding (single products)
 };
 
@@ -26,6 +26,8 @@ struct GemvParams {
 int launch_gemv_streamed(const GemvParams& p, bool dual, bool split, cudaStream_t st);
 // The TMA-fed form for 17..64 tokens: token rows shared by the block's warps through shared memory.
 int launch_gemv_wide(const GemvParams& p, bool dual, bool split, cudaStream_t st);
+// The tcgen05 form (gemv_tc.cu), the default for 1..64 tokens.
+int launch_gemv_tc(const GemvParams& p, bool dual, bool split, cudaStream_t st);
 
 #ifdef __CUDACC__
 __device__ __forceinline__ void mma_s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,

@@ -39,7 +39,7 @@ struct RmsParams {
 __global__ void __launch_bounds__(kThreads) mix_rmsnorm_quant_kernel(RmsParams p) {
   __shared__ double red_d[kThreads / 32];
   __shared__ float red_f[kThreads / 32];
-  grid_dependency_sync();
+  grid_dependency_wait_release();
   const int row = blockIdx.x;
   const __half* x = p.x + row * p.x_row_stride;
   if (p.clear_words != nullptr)
@@ -77,7 +77,7 @@ struct GroupParams {
 };
 
 __global__ void __launch_bounds__(kThreads) mix_group_quant_kernel(GroupParams p) {
-  grid_dependency_sync();
+  grid_dependency_wait_release();
   const int row = blockIdx.x;
   const bool two = p.split < p.cols;
   float m0 = __uint_as_float(p.absmax[row * p.absmax_stride]);
@@ -117,7 +117,7 @@ struct AccParams {
 
 __global__ void __launch_bounds__(kThreads) mix_acc_quant_kernel(AccParams p) {
   __shared__ float red_f[kThreads / 32];
-  grid_dependency_sync();
+  grid_dependency_wait_release();
   const int row = blockIdx.x;
   const int32_t* acc = p.acc + row * p.acc_row_stride;
   const float rs = p.row_scale[row * p.row_scale_stride];

@@ -1,0 +1,58 @@
+"""The default (tcgen05) form of the weight-streaming product: tile edges, remainders of K and tokens, every epilogue."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(m, n, k, dual, split, seed=0, pad=0):
+    g = torch.Generator().manual_seed(seed)
+    ri = lambda *s: torch.randint(-128, 128, s, generator=g, dtype=torch.int8)
+    # rows of the activations lie in a wider tensor, like the latents of a pair
+    wide = ri(m, (2 if split else 1) * k + 16 * pad).cuda()
+    d = dict(a=wide[:, :k], w=ri(n, k).cuda(), sa=(torch.rand(m, generator=g) * 1e-2 + 1e-3).cuda(),
+             ws=(torch.rand(n, generator=g) * 1e-2 + 1e-3).cuda())
+    if dual:
+        d.update(w2=ri(n, k).cuda(), ws2=(torch.rand(n, generator=g) * 1e-2 + 1e-3).cuda())
+    if split:
+        d.update(a2=wide[:, k:2 * k], sa2=(torch.rand(m, generator=g) * 1e-2 + 1e-3).cuda())
+    return d
+
+
+SHAPES = [(1, 16, 16), (3, 48, 80), (4, 128, 128), (5, 144, 256), (16, 1024, 4096), (17, 272, 496), (29, 5504, 512), (32, 64, 2048),
+          (33, 208, 1040), (47, 4096, 384), (48, 112, 2064), (63, 4112, 1024), (64, 2560, 528), (64, 32, 16384)]
+
+
+@pytest.mark.parametrize("m,n,k", SHAPES)
+@pytest.mark.parametrize("kind", ["single", "dual", "split"])
+def test_accumulators_and_results(m, n, k, kind):
+    """int32 sums against float64 (exact: |sum| < 2**53), fp16 results and the all-fp32 epilogue's row maxima bit for bit
+    against the register-fed form, which shares nothing with this one but the epilogue's statement."""
+    from lsvd_b200.ffn import w8a8_gemv
+    dual, split = kind != "single", kind == "split"
+    d = _case(m, n, k, dual, split, seed=m + n, pad=1)
+    kw = dict(w2_q=d["w2"], w2_scale=d["ws2"]) if dual else {}
+    if split:
+        kw.update(a2_q=d["a2"], a2_scale=d["sa2"])
+    res = torch.randn(m, n + 3, device="cuda").half()[:, 1:n + 1] if not dual else None      # odd stride, 2-byte aligned
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    buf = [torch.zeros(m, n + 5, dtype=torch.float16, device="cuda") for _ in range(2)]
+    got = w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], want_acc=True, residual=res, out=buf[0], out_col=3, status_word=status, **kw)
+    want = w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], want_acc=True, residual=res, out=buf[1], out_col=3, form=3, **kw)
+    assert int(status) == 0
+    exact = d["a"].double() @ d["w"].double().t()
+    assert torch.equal(got[1].double(), exact)
+    if dual:
+        a2 = d["a2"] if split else d["a"]
+        assert torch.equal(got[2].double(), a2.double() @ d["w2"].double().t())
+    assert torch.equal(buf[0], buf[1])                                     # untouched border columns included
+    if not dual:
+        o32 = [torch.empty(m, n, device="cuda") for _ in range(2)]
+        w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], want_out=False, out_f32=o32[0])
+        w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], want_out=False, out_f32=o32[1], form=3)
+        assert torch.equal(o32[0], o32[1])
+    words = [torch.zeros(m, 4, dtype=torch.int32, device="cuda") for _ in range(2)]
+    outs = [w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], fp32_swiglu=dual, row_absmax=words[i], absmax_split=16 if n > 16 else 0,
+                      form=3 * i, prefetch_weights=i == 0, **kw)[0] for i in range(2)]
+    assert torch.equal(outs[0], outs[1])
+    assert torch.equal(words[0], words[1])
