@@ -55,6 +55,26 @@ __device__ __forceinline__ int8_t act_code(float x, float s) {
   return static_cast<int8_t>(fminf(fmaxf(y, -128.f), 127.f));
 }
 
+// The same codes without a division per entry.  r = 1 / s correctly rounded (once per row); q0 = x r, its residual
+// x - q0 s exactly in one FMA, and one correction give the correctly rounded quotient (P. Markstein, Computation of
+// elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990); the rounding to an integer is an
+// addition of 1.5 * 2^23, whose low byte is the code.  |x| <= 127 s by the choice of s, so only a NaN needs the clamp (to
+// -128, as fmaxf does in act_code).  An infinite scale would turn finite entries into NaN: such a row divides.
+struct ActCoder {
+  float s, r;
+  bool divide;
+  __device__ __forceinline__ explicit ActCoder(float scale) : s(scale), r(1.0f / scale), divide(!(scale < INFINITY)) {}
+  __device__ __forceinline__ uint32_t low(float x) const {             // the code in the low byte
+    if (divide) return static_cast<uint32_t>(static_cast<uint8_t>(act_code(x, s)));
+    const float q0 = __fmul_rn(x, r);
+    const float y = __fmaf_rn(__fmaf_rn(-q0, s, x), r, q0);
+    return __float_as_uint(__fadd_rn(fmaxf(y, -128.f), 12582912.f));
+  }
+  __device__ __forceinline__ uint32_t four(float a, float b, float c, float d) const {
+    return __byte_perm(__byte_perm(low(a), low(b), 0x0040), __byte_perm(low(c), low(d), 0x0040), 0x5410);
+  }
+};
+
 // One row by one thread block.  `row`: cols floats of shared memory, `red`: 8 floats.  Every thread of the block
 // must call it (block barriers inside); any block size that is a multiple of 32 up to 256.
 __device__ __forceinline__ void act_quant_row(const ActQuantParams& p, int r, float* row, float* red) {
@@ -287,14 +307,15 @@ __device__ __forceinline__ void act_quant_rot4096_row(const ActQuantParams& p, i
   const float s = act_scale_of(amax);
   if (T == 0) p.scale[r] = s;
   // 16 consecutive entries per thread again: one 16-byte store of codes (and two of fp16 values if wanted)
-  __align__(16) int8_t codes[16];
+  const ActCoder coder(s);
+  __align__(16) uint32_t codes[4];
   __align__(16) __half hv[16];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const float v = row[rot_slot(16 * T + i)];
-    codes[i] = act_code(v, s);
-    hv[i] = __float2half_rn(v);
-  }
+  for (int i = 0; i < 16; ++i) e[i] = row[rot_slot(16 * T + i)];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) codes[i] = coder.four(e[4 * i], e[4 * i + 1], e[4 * i + 2], e[4 * i + 3]);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) hv[i] = __float2half_rn(e[i]);
   *reinterpret_cast<uint4*>(p.q + r * p.q_row_stride + 16 * T) = *reinterpret_cast<const uint4*>(codes);
   if (p.x_rot != nullptr) {
     uint4* dst = reinterpret_cast<uint4*>(p.x_rot + static_cast<int64_t>(r) * p.cols + 16 * T);
@@ -379,5 +400,8 @@ __device__ __forceinline__ void mma_f16_16x8x16(float (&d)[4], uint32_t a0, uint
 }
 
 #endif  // __CUDACC__
+
+// One token per block, nb = 64 or 128 and K <= 176 (hadamard_tokens.cu); LSVD_ERR_UNSUPPORTED outside that.
+int launch_hadamard_tokens(const HadQuantParams& p, cudaStream_t st);
 
 }  // namespace lsvd

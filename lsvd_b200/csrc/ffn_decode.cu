@@ -36,6 +36,12 @@ __global__ void __launch_bounds__(256) act_quant_rot4096_kernel(const __grid_con
   act_quant_rot4096_row(p, blockIdx.x, row, red);
 }
 
+__device__ __forceinline__ uint2 codes_of_chunk(const ActCoder& coder, const uint4& v) {
+  const __half2* h = reinterpret_cast<const __half2*>(&v);
+  const float2 a = __half22float2(h[0]), b = __half22float2(h[1]), c = __half22float2(h[2]), d = __half22float2(h[3]);
+  return make_uint2(coder.four(a.x, a.y, b.x, b.y), coder.four(c.x, c.y, d.x, d.y));
+}
+
 // ----------------------------------------------------------------------------------------------
 // per-token quantisation of MANY rows (prefill): one warp per row, the row in registers
 // ----------------------------------------------------------------------------------------------
@@ -98,18 +104,89 @@ __global__ void __launch_bounds__(256, (NCH <= 16 ? 2 : 1)) act_quant_rows_kerne
   amax = warp_max(amax);
   const float s = act_scale_of(amax);
   if (lane == 0) p.scale[r] = s;
+  const ActCoder coder(s);
   uint2* q = reinterpret_cast<uint2*>(p.q + r * p.q_row_stride);
 #pragma unroll
-  for (int c = 0; c < NCH; ++c) {
-    const __half2* h = reinterpret_cast<const __half2*>(&xv[c]);
-    uint32_t w2[2] = {0u, 0u};
+  for (int c = 0; c < NCH; ++c) q[c * 32 + lane] = codes_of_chunk(coder, xv[c]);
+}
+
+// ----------------------------------------------------------------------------------------------
+// per-token quantisation of a decode batch: one block per row, the row in registers
+// ----------------------------------------------------------------------------------------------
+// At a few rows the quantiser is a latency: launch, one load, the reductions, one store.  A thread holds NV 16-byte chunks
+// of the row and of the norm weight, all requested at once; each reduction is a warp shuffle, one block barrier and a
+// second shuffle.  act_quant_kernel passes the row through shared memory with scalar loops and five barriers more:
+// RMSNorm + A8 of 16 x 4096 took 11.5 us there.  No rotation, no fp32 input, no fake-quantised output.
+template <int NV>
+__global__ void __launch_bounds__(1024) act_quant_block_kernel(const __grid_constant__ ActQuantParams p) {
+  __shared__ float red[2][32];
+  grid_dependency_wait_release();
+  const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int chunks = p.cols >> 3;
+  const uint4* x = reinterpret_cast<const uint4*>(p.x + r * p.x_row_stride);
+  const uint4* w = reinterpret_cast<const uint4*>(p.norm_weight);
+  uint4 xv[NV], wv[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int c = threadIdx.x + v * blockDim.x;
+    xv[v] = wv[v] = make_uint4(0u, 0u, 0u, 0u);
+    if (c < chunks) {
+      xv[v] = __ldcg(x + c);
+      if (p.norm_weight != nullptr) wv[v] = __ldg(w + c);
+    }
+  }
+  if (p.norm_weight != nullptr) {
+    float ss = 0.f;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const __half2* h = reinterpret_cast<const __half2*>(&xv[v]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __half22float2(h[e]);
+        ss = fmaf(f.x, f.x, ss);
+        ss = fmaf(f.y, f.y, ss);
+      }
+    }
+    ss = warp_sum(ss);
+    if (lane == 0) red[0][warp] = ss;
+    __syncthreads();
+    const float inv = rsqrtf(warp_sum(lane < warps ? red[0][lane] : 0.f) / static_cast<float>(p.cols) + p.norm_eps);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const int c = threadIdx.x + v * blockDim.x;
+      __half2* h = reinterpret_cast<__half2*>(&xv[v]);
+      const __half2* wh = reinterpret_cast<const __half2*>(&wv[v]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __half22float2(h[e]), g = __half22float2(wh[e]);
+        // fp32 statistics, the normalised value rounded to fp16, then an fp16 product with the weight (act_quant_row)
+        const __half a = __float2half_rn(f.x * inv), b = __float2half_rn(f.y * inv);
+        h[e] = __halves2half2(__float2half_rn(__half2float(a) * g.x), __float2half_rn(__half2float(b) * g.y));
+      }
+      if (p.x_rot != nullptr && c < chunks) reinterpret_cast<uint4*>(p.x_rot + static_cast<int64_t>(r) * p.cols)[c] = xv[v];
+    }
+  }
+  float amax = 0.f;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const __half2* h = reinterpret_cast<const __half2*>(&xv[v]);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float2 f = __half22float2(h[e]);
-      w2[e >> 1] |= static_cast<uint32_t>(static_cast<uint8_t>(act_code(f.x, s))) << (16 * (e & 1));
-      w2[e >> 1] |= static_cast<uint32_t>(static_cast<uint8_t>(act_code(f.y, s))) << (16 * (e & 1) + 8);
+      amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
     }
-    q[c * 32 + lane] = make_uint2(w2[0], w2[1]);
+  }
+  amax = warp_max(amax);
+  if (lane == 0) red[1][warp] = amax;
+  __syncthreads();
+  const float s = act_scale_of(warp_max(lane < warps ? red[1][lane] : 0.f));
+  if (threadIdx.x == 0) p.scale[r] = s;
+  const ActCoder coder(s);
+  uint2* q = reinterpret_cast<uint2*>(p.q + r * p.q_row_stride);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int c = threadIdx.x + v * blockDim.x;
+    if (c < chunks) q[c] = codes_of_chunk(coder, xv[v]);
   }
 }
 
@@ -448,146 +525,6 @@ __global__ void __launch_bounds__(256) hadamard_quant_kernel(const __grid_consta
 }
 
 // ----------------------------------------------------------------------------------------------
-// The same rotation + quantisation for many tokens (prefill): one block per token, built for throughput
-// ----------------------------------------------------------------------------------------------
-// nb = 64.  A warp rotates four 64-entry blocks at a time: a lane holds eight consecutive entries of one block
-// (one 16-byte load), does the strides 1, 2, 4 in registers and the strides 8, 16, 32 with three rounds of
-// shuffles: the same additions in the same order as the butterfly loop.  The had_K product and the fp16
-// roundings are those of hadamard_quant_kernel; the int8 codes are staged in shared memory and leave as
-// 16-byte stores.
-constexpr int kRowsNb = 64;
-
-__global__ void __launch_bounds__(512) hadamard_quant_rows_kernel(const __grid_constant__ HadQuantParams p) {
-  extern __shared__ __align__(16) uint8_t smem_raw[];
-  __shared__ float red[16];
-  const int K = p.K, ld = p.ld;                              // ld = Kp + 10 halves here
-  __half* Tt = reinterpret_cast<__half*>(smem_raw);           // [64][ld]: column j of every rotated block
-  uint8_t* Tq = smem_raw;                                     // [Kp][80] int8 codes, after the product (same bytes)
-  const int r = blockIdx.x;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nw = blockDim.x >> 5;                              // one warp per 16-row tile of had_K: Kp / 16 warps
-  const __half* xg = p.x + r * p.x_row_stride;
-
-  // columns K .. Kp of Tt meet zero entries of had_K in the product: they must hold numbers, not leftovers
-  for (int i = threadIdx.x; i < kRowsNb * (p.Kp - K); i += blockDim.x) {
-    const int j = i / (p.Kp - K), k = K + (i - j * (p.Kp - K));
-    Tt[j * ld + k] = __float2half_rn(0.f);
-  }
-  {
-    const int sub = lane & 7, quad = lane >> 3;
-    constexpr int kMaxIter = 4;                     // K / 4 groups of four blocks over Kp / 16 warps: at most 4 each
-    uint4 xv[kMaxIter];
-#pragma unroll
-    for (int it = 0; it < kMaxIter; ++it) {         // every load of this lane in flight before the first use
-      const int k = (warp + it * nw) * 4 + quad;
-      xv[it] = make_uint4(0u, 0u, 0u, 0u);
-      if (k < K) xv[it] = __ldg(reinterpret_cast<const uint4*>(xg + k * kRowsNb) + sub);
-    }
-#pragma unroll
-    for (int it = 0; it < kMaxIter; ++it) {
-      const int k = (warp + it * nw) * 4 + quad;
-      if ((warp + it * nw) * 4 >= K) break;
-      float e[8];
-      {
-        const __half2* h2 = reinterpret_cast<const __half2*>(&xv[it]);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 f = __half22float2(h2[i]);
-          e[2 * i] = f.x;
-          e[2 * i + 1] = f.y;
-        }
-      }
-#pragma unroll
-      for (int h = 1; h < 8; h <<= 1)
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if ((i & h) == 0) {
-            const float a = e[i], b = e[i + h];
-            e[i] = a + b;
-            e[i + h] = a - b;
-          }
-#pragma unroll
-      for (int h = 1; h < 8; h <<= 1)              // strides 8, 16, 32 <-> lane bits 0, 1, 2
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float o = __shfl_xor_sync(0xffffffffu, e[i], h);
-          e[i] = (sub & h) ? o - e[i] : e[i] + o;
-        }
-      if (k < K) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) Tt[(sub * 8 + i) * ld + k] = __float2half_rn(e[i] * p.rot_scale);
-      }
-    }
-  }
-  __syncthreads();
-
-  // ---- had_K product: warp w owns m tile w ----
-  const int g = lane >> 2, t = lane & 3;
-  const int tiles = p.Kp >> 4;
-  const int mt = warp;
-  float d[8][4];
-  float amax = 0.f;
-#pragma unroll
-  for (int ni = 0; ni < 8; ++ni)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) d[ni][c] = 0.f;
-  {
-    const uint4* ap = p.packed + (static_cast<int64_t>(mt) * tiles) * 32 + lane;
-    uint4 af[4];                                 // four fragments of had_K in flight
-#pragma unroll
-    for (int u = 0; u < 4; ++u) af[u] = u < tiles ? __ldg(ap + u * 32) : make_uint4(0u, 0u, 0u, 0u);
-    for (int kt0 = 0; kt0 < tiles; kt0 += 4) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int kt = kt0 + u;
-        if (kt < tiles) {
-          const uint4 a4 = af[u];
-          if (kt + 4 < tiles) af[u] = __ldg(ap + (kt + 4) * 32);
-#pragma unroll
-          for (int ni = 0; ni < 8; ++ni) {
-            const __half* brow = Tt + (ni * 8 + g) * ld + kt * 16 + 2 * t;
-            const uint32_t b0 = *reinterpret_cast<const uint32_t*>(brow);
-            const uint32_t b1 = *reinterpret_cast<const uint32_t*>(brow + 8);
-            mma_f16_16x8x16(d[ni], a4.x, a4.y, a4.z, a4.w, b0, b1);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int ni = 0; ni < 8; ++ni)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        d[ni][c] = __half2float(__float2half_rn(d[ni][c]));        // the reference's fp16 result
-        if (mt * 16 + g + 8 * (c >> 1) < K) amax = fmaxf(amax, fabsf(d[ni][c]));
-      }
-  }
-  amax = block_max(amax, red);                // its barriers also end every warp's reads of Tt
-  const float s = act_scale_of(amax);
-  if (threadIdx.x == 0) p.scale[r] = s;
-
-  // ---- quantise into shared memory (rows of 80 bytes: conflict-free 2-byte stores, 16-byte aligned rows) ----
-#pragma unroll
-  for (int ni = 0; ni < 8; ++ni)
-#pragma unroll
-    for (int hf = 0; hf < 2; ++hf) {
-      const int row = mt * 16 + g + 8 * hf;
-      const uint16_t packed = static_cast<uint16_t>(static_cast<uint8_t>(act_code(d[ni][2 * hf], s))) |
-                              (static_cast<uint16_t>(static_cast<uint8_t>(act_code(d[ni][2 * hf + 1], s))) << 8);
-      *reinterpret_cast<uint16_t*>(Tq + row * 80 + ni * 8 + 2 * t) = packed;
-    }
-  __syncthreads();
-  int8_t* q = p.q + r * p.q_row_stride;
-  if ((reinterpret_cast<uintptr_t>(q) & 15) == 0) {
-    for (int i = threadIdx.x; i < K * 4; i += blockDim.x) {
-      const int row = i >> 2, c = i & 3;
-      reinterpret_cast<uint4*>(q)[i] = *reinterpret_cast<const uint4*>(Tq + row * 80 + c * 16);
-    }
-  } else {
-    for (int i = threadIdx.x; i < K * kRowsNb; i += blockDim.x) q[i] = static_cast<int8_t>(Tq[(i >> 6) * 80 + (i & 63)]);
-  }
-}
-
-// ----------------------------------------------------------------------------------------------
 // weight-streaming W8A8 product
 // ----------------------------------------------------------------------------------------------
 constexpr int kGemvWarps = 8;
@@ -826,6 +763,15 @@ extern "C" int lsvd_act_quant(const lsvd_act_quant_args* a, void* stream) {
       return LSVD_OK;
     }
   }
+  // any other row of whole, aligned 16-byte chunks without a rotation: at most two chunks per thread
+  if (!rotate && a->x_f32 == nullptr && p.fake == nullptr && p.vec8 && (p.x_rot == nullptr || (p.norm_weight != nullptr && aligned(p.x_rot, 16))) &&
+      (p.norm_weight == nullptr || aligned(p.norm_weight, 16))) {
+    const int chunks = a->cols / 8;
+    const int threads = std::min(1024, (chunks + 31) / 32 * 32);
+    LSVD_CUDA_TRY(launch_chained(chunks <= 1024 ? act_quant_block_kernel<1> : act_quant_block_kernel<2>, dim3(a->rows), dim3(threads), 0,
+                                 static_cast<cudaStream_t>(stream), 1, true, p));
+    return LSVD_OK;
+  }
   const int smem = a->cols * 4;
   if (smem > 48 * 1024) LSVD_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(act_quant_kernel), smem));
   LSVD_CUDA_TRY(launch_chained(act_quant_kernel, dim3(a->rows), dim3(256), smem, static_cast<cudaStream_t>(stream), 1, true, p));
@@ -964,6 +910,12 @@ extern "C" int lsvd_hadamard_quant(const lsvd_hadamard_quant_args* a, void* stre
   p.nb = nb;
   p.Kp = (a->K + 15) / 16 * 16;
   p.ld = p.Kp + 8;
+  p.rot_scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(a->cols)));
+  p.x_vec16 = (aligned(a->x, 16) && (a->x_row_stride % 8) == 0 && (a->cols % 8) == 0) ? 1 : 0;
+  {
+    const int rc = launch_hadamard_tokens(p, static_cast<cudaStream_t>(stream));
+    if (rc != LSVD_ERR_UNSUPPORTED) return rc;
+  }
   const int ntiles = nb / 8;
   // Few tokens: a cluster of up to 8 blocks per token shortens the critical path.  Many tokens: one block (two
   // for nb = 128) per token keeps every SM busy without the cluster's redundant staging.
@@ -975,18 +927,7 @@ extern "C" int lsvd_hadamard_quant(const lsvd_hadamard_quant_args* a, void* stre
     p.cluster = ntiles < 8 ? ntiles : 8;
   }
   p.ntile_per = ntiles / p.cluster;
-  p.rot_scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(a->cols)));
   const int smem = (p.ntile_per * 8 * p.ld + a->cols) * 2;
-  p.x_vec16 = (aligned(a->x, 16) && (a->x_row_stride % 8) == 0 && (a->cols % 8) == 0) ? 1 : 0;
-  if (many && nb == kRowsNb && a->y == nullptr && p.x_vec16 && (a->x_row_stride % 8) == 0) {
-    p.ld = p.Kp + 10;
-    const int smem_rows = std::max(kRowsNb * p.ld * 2, p.Kp * 80);
-    if (smem_rows > 48 * 1024)
-      LSVD_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(hadamard_quant_rows_kernel), smem_rows));
-    LSVD_CUDA_TRY(launch_chained(hadamard_quant_rows_kernel, dim3(static_cast<unsigned>(a->rows)), dim3(p.Kp * 2), smem_rows,
-                                 static_cast<cudaStream_t>(stream), 1, true, p));
-    return LSVD_OK;
-  }
   void (*kern)(HadQuantParams) = p.ntile_per <= 2 ? hadamard_quant_kernel<2> : hadamard_quant_kernel<8>;
   if (smem > 48 * 1024) LSVD_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
   LSVD_CUDA_TRY(launch_chained(kern, dim3(static_cast<unsigned>(a->rows * p.cluster)), dim3(256), smem,
