@@ -55,6 +55,26 @@ __device__ __forceinline__ int8_t act_code(float x, float s) {
   return static_cast<int8_t>(fminf(fmaxf(y, -128.f), 127.f));
 }
 
+// Two fp32 operations in one instruction (sm_100): each lane is the single rounded operation.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+
 // The same codes without a division per entry.  r = 1 / s correctly rounded (once per row); q0 = x r, its residual
 // x - q0 s exactly in one FMA, and one correction give the correctly rounded quotient (P. Markstein, Computation of
 // elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990); the rounding to an integer is an
@@ -62,16 +82,20 @@ __device__ __forceinline__ int8_t act_code(float x, float s) {
 // -128, as fmaxf does in act_code).  An infinite scale would turn finite entries into NaN: such a row divides.
 struct ActCoder {
   float s, r;
-  bool divide;
+  bool divide;                                   // the same for the whole row
   __device__ __forceinline__ explicit ActCoder(float scale) : s(scale), r(1.0f / scale), divide(!(scale < INFINITY)) {}
-  __device__ __forceinline__ uint32_t low(float x) const {             // the code in the low byte
-    if (divide) return static_cast<uint32_t>(static_cast<uint8_t>(act_code(x, s)));
-    const float q0 = __fmul_rn(x, r);
-    const float y = __fmaf_rn(__fmaf_rn(-q0, s, x), r, q0);
-    return __float_as_uint(__fadd_rn(fmaxf(y, -128.f), 12582912.f));
+  // the codes of two entries in bytes 0 and 1 (the upper bytes hold leftovers of the second)
+  template <bool kDivide>
+  __device__ __forceinline__ uint32_t pair(float2 v) const {
+    if (kDivide) return static_cast<uint32_t>(static_cast<uint8_t>(act_code(v.x, s))) | (static_cast<uint32_t>(static_cast<uint8_t>(act_code(v.y, s))) << 8);
+    const float2 q0 = mul2(v, make_float2(r, r));
+    float2 y = fma2(fma2(q0, make_float2(-s, -s), v), make_float2(r, r), q0);
+    y = add2(make_float2(fmaxf(y.x, -128.f), fmaxf(y.y, -128.f)), make_float2(12582912.f, 12582912.f));
+    return __byte_perm(__float_as_uint(y.x), __float_as_uint(y.y), 0x0040);
   }
-  __device__ __forceinline__ uint32_t four(float a, float b, float c, float d) const {
-    return __byte_perm(__byte_perm(low(a), low(b), 0x0040), __byte_perm(low(c), low(d), 0x0040), 0x5410);
+  template <bool kDivide>
+  __device__ __forceinline__ uint32_t four(float2 a, float2 b) const {
+    return __byte_perm(pair<kDivide>(a), pair<kDivide>(b), 0x5410);
   }
 };
 
@@ -313,7 +337,10 @@ __device__ __forceinline__ void act_quant_rot4096_row(const ActQuantParams& p, i
 #pragma unroll
   for (int i = 0; i < 16; ++i) e[i] = row[rot_slot(16 * T + i)];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) codes[i] = coder.four(e[4 * i], e[4 * i + 1], e[4 * i + 2], e[4 * i + 3]);
+  for (int i = 0; i < 4; ++i) {
+    const float2 a = make_float2(e[4 * i], e[4 * i + 1]), b = make_float2(e[4 * i + 2], e[4 * i + 3]);
+    codes[i] = coder.divide ? coder.four<true>(a, b) : coder.four<false>(a, b);
+  }
 #pragma unroll
   for (int i = 0; i < 16; ++i) hv[i] = __float2half_rn(e[i]);
   *reinterpret_cast<uint4*>(p.q + r * p.q_row_stride + 16 * T) = *reinterpret_cast<const uint4*>(codes);

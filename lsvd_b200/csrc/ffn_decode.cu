@@ -39,7 +39,8 @@ __global__ void __launch_bounds__(256) act_quant_rot4096_kernel(const __grid_con
 __device__ __forceinline__ uint2 codes_of_chunk(const ActCoder& coder, const uint4& v) {
   const __half2* h = reinterpret_cast<const __half2*>(&v);
   const float2 a = __half22float2(h[0]), b = __half22float2(h[1]), c = __half22float2(h[2]), d = __half22float2(h[3]);
-  return make_uint2(coder.four(a.x, a.y, b.x, b.y), coder.four(c.x, c.y, d.x, d.y));
+  if (coder.divide) return make_uint2(coder.four<true>(a, b), coder.four<true>(c, d));
+  return make_uint2(coder.four<false>(a, b), coder.four<false>(c, d));
 }
 
 // ----------------------------------------------------------------------------------------------
