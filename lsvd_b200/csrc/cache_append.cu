@@ -110,82 +110,182 @@ __global__ void __launch_bounds__(128) cache_append_kernel(const __grid_constant
   if (lane == 0) *scale_unit(p, s, dest, h) = s16;
 }
 
-// Prefill-sized calls.  Units are ordered head by head (all tokens of head 0 of K, then head 1, ...), so a warp works
-// on ONE head and its lanes can be dealt by that head's rank: L = 2, 4, 8 or 16 lanes per (token, head) unit for ranks
-// up to 16, 32, 64, 128, a lane owning 8 consecutive entries (16-byte load, 8-byte store), 32 / L tokens per warp.
-// The one-unit-per-warp kernel above issues two to sixteen times as many warp instructions per byte, and at these
-// sizes instruction issue, not memory, is what bounds it.  Same arithmetic, so the same bits.
-struct WideTable {
-  int32_t warp_begin[2 * LSVD_MAX_HEADS + 1];   // first warp of every (side, head) segment, in launch order
-  int32_t seg_side_head[2 * LSVD_MAX_HEADS];    // side * LSVD_MAX_HEADS + head
-  int32_t nseg;
-};
+// Prefill-sized calls.  A thread owns 16 consecutive latents of one head (a chunk; ranks are multiples of 16) in four tokens
+// at a time and keeps that column for all its tokens, so the head look-up, offsets and strides are paid once per block and a
+// block reads whole token rows: 4 x 32 bytes per thread in flight, contiguous across the block, and one 16-byte store of
+// codes per chunk.  The chunks of a head exchange their maxima through shared memory, four tokens per 8-byte word (one
+// barrier per four tokens: the words are double-buffered).  The arithmetic is packed: quotients two at a time in fp32 (as
+// in quantise_one), everything after the rounding to fp16 in fp16 pairs -- adding 1536 rounds to an integer half to even
+// and leaves the code in the low byte -- about seven instructions per latent.
+// 32 768 tokens x (2048 + 2048) latents, 402 MB: 115 us, 3.5 TB/s.  Head-by-head order with eight
+// latents per lane took 224 us (issue bound, and 32..256 bytes of a row at a time).
+constexpr int kRowTokens = 4;
 
+// Four codes of (x - already loaded - as two half pairs).  r = 1 / s correctly rounded; a scale that is not finite takes
+// quantise_one, whose NaN rules the packed form does not reproduce for the triton rounding.
 template <int kRounding>
-__global__ void __launch_bounds__(128) cache_append_wide_kernel(const __grid_constant__ AppendParams p,
-                                                                const __grid_constant__ WideTable w) {
-  grid_dependency_sync();
-  const int lane = threadIdx.x & 31;
-  const int warp_id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (warp_id >= w.warp_begin[w.nseg]) return;
-  int lo_seg = 0, hi_seg = w.nseg;                   // last segment whose first warp is <= warp_id
-  while (hi_seg - lo_seg > 1) {
-    const int mid = (lo_seg + hi_seg) >> 1;
-    if (w.warp_begin[mid] <= warp_id) lo_seg = mid; else hi_seg = mid;
-  }
-  const int side = w.seg_side_head[lo_seg] / LSVD_MAX_HEADS, h = w.seg_side_head[lo_seg] % LSVD_MAX_HEADS;
-  const AppendSide& s = p.side[side];
-  const int r0 = s.rank_off[h];
-  const int rank = s.rank_off[h + 1] - r0;
-  const int lg = rank <= 16 ? 1 : (rank <= 32 ? 2 : (rank <= 64 ? 3 : 4));     // log2 of the lanes per unit
-  const int sub = lane & ((1 << lg) - 1);
-  const int t = (warp_id - w.warp_begin[lo_seg]) * (32 >> lg) + (lane >> lg);
-  const bool live = t < p.num_tokens;
-  const int i0 = sub * 8;
-  const bool active = live && i0 < rank;
-
-  float x[8];
+__device__ __forceinline__ uint32_t quantise_four(uint32_t w0, uint32_t w1, float s, float r) {
+  uint32_t out[2];
+  const uint32_t w[2] = {w0, w1};
 #pragma unroll
-  for (int j = 0; j < 8; ++j) x[j] = 0.f;
-  if (active) {
-    const uint4 raw = *reinterpret_cast<const uint4*>(s.latent + static_cast<int64_t>(t) * s.token_stride + s.head_off[h] + i0);
-    const __half2* h2 = reinterpret_cast<const __half2*>(&raw);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      x[2 * j] = __low2float(h2[j]);
-      x[2 * j + 1] = __high2float(h2[j]);
+  for (int i = 0; i < 2; ++i) {
+    const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+    const float2 q0 = mul2(x, make_float2(r, r));
+    const float2 y = fma2(fma2(q0, make_float2(-s, -s), x), make_float2(r, r), q0);
+    if (kRounding == LSVD_ROUND_TORCH) {
+      // |y| <= 128 by the choice of the scale; a NaN becomes -128
+      __half2 h = __float22half2_rn(y);
+      h = __hmin2(__hmax2(h, __float2half2_rn(-128.f)), __float2half2_rn(127.f));
+      h = __hadd2(h, __float2half2_rn(1536.f));
+      out[i] = *reinterpret_cast<const uint32_t*>(&h);           // codes in bytes 0 and 2
+    } else {
+      // trunc(y +- 0.5): floor of |y| + 0.5 by an addition rounded towards zero, the sign put back; a NaN becomes 0
+      const int a = static_cast<int>(__float_as_uint(__fadd_rz(fmaxf(fabsf(y.x) + 0.5f, 0.f), 8388608.f)) & 0xffu);
+      const int b = static_cast<int>(__float_as_uint(__fadd_rz(fmaxf(fabsf(y.y) + 0.5f, 0.f), 8388608.f)) & 0xffu);
+      const int ca = y.x < 0.f ? -a : min(a, 127), cb = y.y < 0.f ? -b : min(b, 127);
+      out[i] = __byte_perm(static_cast<uint32_t>(ca), static_cast<uint32_t>(cb), 0x5410);
     }
   }
-  float amax = 0.f;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(x[j]));
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1)
-    if (o < (1 << lg)) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));     // lg is uniform in the warp
-  __half s16 = __float2half_rn(amax * 0.0078125f);
-  const __half floor16 = __float2half_rn(1e-4f);
-  if (__half2float(s16) < __half2float(floor16)) s16 = floor16;
-  const float sf = __half2float(s16);
-  const float rsf = __frcp_rn(sf);
-  if (!live) return;
-  const int dest = p.dest_loc[t];
-  if (dest < 0 || dest >= p.num_slots) {
-    if (sub == 0) report_status(p.status_word, LSVD_ERR_BOUNDS);
-    return;
-  }
-  if (active) {
-    uint32_t lo = 0, hi = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      lo |= (static_cast<uint32_t>(quantise_one<kRounding>(x[j], sf, rsf)) & 0xffu) << (8 * j);
-      hi |= (static_cast<uint32_t>(quantise_one<kRounding>(x[4 + j], sf, rsf)) & 0xffu) << (8 * j);
-    }
-    *reinterpret_cast<uint2*>(cache_unit(p, s, dest, r0, rank) + i0) = make_uint2(lo, hi);
-  }
-  if (sub == 0) *scale_unit(p, s, dest, h) = s16;
+  return __byte_perm(out[0], out[1], 0x6420);
 }
 
-// The wide kernel's accesses: 16-byte loads of the latents, 8-byte stores of the codes.
+// kBulk: the next four token rows travel by bulk copies (one per token, heads back to back in memory) while these are
+// quantised; the barrier of the maxima also tells that everybody has read the stage.  Loads straight into registers -- heads
+// at their own offsets, or rows too wide for two stages -- leave the memory idle while a block computes (128 us instead of
+// the figure above); the same prefetch by 16-byte cp.async per thread took 146 us.
+template <int kRounding, bool kBulk>
+__global__ void __launch_bounds__(1024) cache_append_rows_kernel(const __grid_constant__ AppendParams p, const int first_side) {
+  extern __shared__ __align__(16) uint8_t rows_smem[];
+  uint2* amax_s = reinterpret_cast<uint2*>(rows_smem);  // [2][blockDim]: maxima of a chunk, one half per token
+  uint8_t* stage = rows_smem + 2 * blockDim.x * sizeof(uint2);         // [2][kRowTokens] token rows
+  __shared__ uint64_t full[2];
+  const AppendSide& s = p.side[first_side + blockIdx.y];
+  const int c = threadIdx.x, chunks = s.rank_off[p.num_heads] >> 4;
+  int lo = 0, hi = p.num_heads;                         // last head whose first chunk is <= c
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if ((s.rank_off[mid] >> 4) <= c) lo = mid; else hi = mid;
+  }
+  const int r0 = s.rank_off[lo], rank = s.rank_off[lo + 1] - r0;
+  const int c0 = r0 >> 4, n = rank >> 4;
+  const bool on = c < chunks;
+  const __half* src = s.latent + s.head_off[lo] + (c - c0) * 16;
+  const int row_bytes = s.rank_off[p.num_heads] * 2;
+  if (kBulk && threadIdx.x == 0) {
+    mbar_init(&full[0], 1);
+    mbar_init(&full[1], 1);
+    fence_mbar_init();
+  }
+  if (kBulk) __syncthreads();
+  int8_t* dst = p.head_major ? s.cache + static_cast<int64_t>(r0) * p.num_slots + (c - c0) * 16 : s.cache + c * 16;
+  const int64_t dst_stride = p.head_major ? rank : s.cache_row_stride;
+  __half* sdst = s.scale + (p.head_major ? static_cast<int64_t>(lo) * p.num_slots : lo);
+  const int64_t s_stride = p.head_major ? 1 : s.scale_row_stride;
+  const bool st16 = ((reinterpret_cast<uintptr_t>(s.cache) | static_cast<uintptr_t>(dst_stride)) & 15) == 0 || p.head_major;
+  grid_dependency_sync();
+
+  auto fetch = [&](int t0, int b) {                     // one thread
+    const int n_tok = min(kRowTokens, p.num_tokens - t0);
+    if (n_tok <= 0) return;
+    mbar_arrive_expect_tx(&full[b], n_tok * row_bytes);
+    for (int j = 0; j < n_tok; ++j)
+      bulk_g2s(stage + (b * kRowTokens + j) * row_bytes, s.latent + s.head_off[0] + static_cast<int64_t>(t0 + j) * s.token_stride, row_bytes, &full[b]);
+  };
+  const int step = gridDim.x * kRowTokens;
+  if (kBulk && threadIdx.x == 0) {
+    fetch(blockIdx.x * kRowTokens, 0);
+    fetch(blockIdx.x * kRowTokens + step, 1);
+  }
+  int buf = 0, round = 0;
+  for (int t0 = blockIdx.x * kRowTokens; t0 < p.num_tokens; t0 += step, buf ^= 1, ++round) {
+    uint4 x[kRowTokens][2];
+    int dest[kRowTokens];
+#pragma unroll
+    for (int j = 0; j < kRowTokens; ++j) dest[j] = t0 + j < p.num_tokens ? p.dest_loc[t0 + j] : -1;
+    const bool late = kBulk && !mbar_wait_bounded(&full[buf], (round >> 1) & 1);
+#pragma unroll
+    for (int j = 0; j < kRowTokens; ++j) {
+      const bool in = t0 + j < p.num_tokens;
+      x[j][0] = x[j][1] = make_uint4(0u, 0u, 0u, 0u);
+      if (in && on) {
+        const uint4* v = kBulk ? reinterpret_cast<const uint4*>(stage + (buf * kRowTokens + j) * row_bytes + c * 32)
+                               : reinterpret_cast<const uint4*>(src + static_cast<int64_t>(t0 + j) * s.token_stride);
+        x[j][0] = v[0];
+        x[j][1] = v[1];
+      }
+      if (in && (dest[j] < 0 || dest[j] >= p.num_slots)) {
+        if (c == 0) report_status(p.status_word, LSVD_ERR_BOUNDS);
+        dest[j] = -1;
+      }
+    }
+    __half m[kRowTokens];
+#pragma unroll
+    for (int j = 0; j < kRowTokens; ++j) {
+      const __half2* h = reinterpret_cast<const __half2*>(x[j]);
+      __half2 top = __float2half2_rn(0.f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) top = __hmax2(top, __habs2(h[e]));
+      m[j] = __hmax(__low2half(top), __high2half(top));
+    }
+    uint2* am = amax_s + buf * blockDim.x;
+    {
+      const __half2 a = __halves2half2(m[0], m[1]), b = __halves2half2(m[2], m[3]);
+      am[c] = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+    }
+    if (kBulk) {
+      if (__syncthreads_or(late)) {                     // a copy did not arrive: nobody goes on
+        if (threadIdx.x == 0) {
+          report_status(p.status_word, LSVD_ERR_TIMEOUT);
+          mbar_wait_bounded(&full[buf], (round >> 1) & 1);        // this block's copies, before its shared memory goes
+          if (t0 + step < p.num_tokens) mbar_wait_bounded(&full[buf ^ 1], ((round + 1) >> 1) & 1);
+        }
+        return;
+      }
+      if (threadIdx.x == 0) fetch(t0 + 2 * step, buf);
+    } else {
+      __syncthreads();
+    }
+    __half2 top[2] = {__float2half2_rn(0.f), __float2half2_rn(0.f)};
+    if (on) {
+      for (int k = 0; k < n; ++k) {
+        const uint2 w = am[c0 + k];
+        top[0] = __hmax2(top[0], *reinterpret_cast<const __half2*>(&w.x));
+        top[1] = __hmax2(top[1], *reinterpret_cast<const __half2*>(&w.y));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kRowTokens; ++j) {
+      if (!on || dest[j] < 0) continue;
+      // absmax is an fp16 value; / 128 in fp16 is one rounding of the exact quotient
+      const float amax = j & 1 ? __high2float(top[j >> 1]) : __low2float(top[j >> 1]);
+      __half s16 = __float2half_rn(amax * 0.0078125f);
+      const __half floor16 = __float2half_rn(1e-4f);
+      if (__half2float(s16) < __half2float(floor16)) s16 = floor16;
+      const float sf = __half2float(s16);
+      const float r = __frcp_rn(sf);
+      uint4 q;
+      if (kRounding == LSVD_ROUND_TORCH || sf < INFINITY) {
+        q = make_uint4(quantise_four<kRounding>(x[j][0].x, x[j][0].y, sf, r), quantise_four<kRounding>(x[j][0].z, x[j][0].w, sf, r),
+                       quantise_four<kRounding>(x[j][1].x, x[j][1].y, sf, r), quantise_four<kRounding>(x[j][1].z, x[j][1].w, sf, r));
+      } else {
+        __align__(16) int8_t codes[16];
+        const __half* h = reinterpret_cast<const __half*>(x[j]);
+        for (int e = 0; e < 16; ++e) codes[e] = static_cast<int8_t>(quantise_one<kRounding>(__half2float(h[e]), sf, r));
+        q = *reinterpret_cast<const uint4*>(codes);
+      }
+      int8_t* d = dst + static_cast<int64_t>(dest[j]) * dst_stride;
+      if (st16) {
+        *reinterpret_cast<uint4*>(d) = q;
+      } else {
+        reinterpret_cast<uint2*>(d)[0] = make_uint2(q.x, q.y);
+        reinterpret_cast<uint2*>(d)[1] = make_uint2(q.z, q.w);
+      }
+      if (c == c0) sdst[static_cast<int64_t>(dest[j]) * s_stride] = s16;
+    }
+  }
+}
+
+// The rows kernel's accesses: 16-byte loads of the latents, stores of at least 8 bytes of the codes.
 static bool side_is_wide_ok(const lsvd_append_tensor& t, int num_heads, bool head_major) {
   if (!aligned(t.latent, 16) || (t.token_stride % 8) != 0 || !aligned(t.cache, 8) || (!head_major && (t.cache_row_stride % 8) != 0)) return false;
   for (int h = 0; h < num_heads; ++h) {
@@ -281,33 +381,35 @@ extern "C" int lsvd_cache_append(const lsvd_append_args* a, void* stream) {
   const int64_t units = static_cast<int64_t>(a->num_tokens) * a->num_heads * sides;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int warps_per_block = 4;
-  bool wide = units >= 32768;
+  // One warp per unit up to here: 32 ragged heads, K and V, 64 / 128 / 256 tokens take 2.6 / 3.4 / 5.7 us that way and
+  // 3.1 / 3.2 / 3.3 us in the row form.
+  bool wide = units >= 8192;
   for (int sd = 0; sd < 2 && wide; ++sd) {
     if (((p.side_mask >> sd) & 1) == 0) continue;
     wide = side_is_wide_ok(sd == 0 ? a->k : a->v, a->num_heads, p.head_major != 0);
   }
   if (wide) {
-    WideTable wt{};
-    int64_t warps = 0;
-    for (int sd = 0; sd < 2; ++sd) {
+    int chunks = 0;
+    for (int sd = 0; sd < 2; ++sd)
+      if ((p.side_mask >> sd) & 1) chunks = std::max(chunks, static_cast<int>((sd == 0 ? a->k : a->v).rank_off[a->num_heads] / 16));
+    const int threads = (chunks + 31) / 32 * 32;
+    const int groups = (a->num_tokens + kRowTokens - 1) / kRowTokens;
+    bool ahead = 16 * chunks * 2 * kRowTokens * 2 <= 96 * 1024;
+    for (int sd = 0; sd < 2 && ahead; ++sd) {
       if (((p.side_mask >> sd) & 1) == 0) continue;
-      const lsvd_append_tensor& t = sd == 0 ? a->k : a->v;
-      for (int h = 0; h < a->num_heads; ++h) {
-        const int rank = t.rank_off[h + 1] - t.rank_off[h];
-        const int lanes = rank <= 16 ? 2 : (rank <= 32 ? 4 : (rank <= 64 ? 8 : 16));
-        const int per_warp = 32 / lanes;
-        wt.warp_begin[wt.nseg] = static_cast<int32_t>(warps);
-        wt.seg_side_head[wt.nseg] = sd * LSVD_MAX_HEADS + h;
-        ++wt.nseg;
-        warps += (a->num_tokens + per_warp - 1) / per_warp;
-      }
+      const AppendSide& side = p.side[sd];
+      ahead = aligned(side.latent + side.head_off[0], 16);
+      for (int h = 0; h < a->num_heads && ahead; ++h) ahead = side.head_off[h] - side.head_off[0] == side.rank_off[h];
     }
-    if (warps > 0x7fffffffLL - 8) return LSVD_ERR_UNSUPPORTED;
-    wt.warp_begin[wt.nseg] = static_cast<int32_t>(warps);
-    const int64_t blocks = (warps + warps_per_block - 1) / warps_per_block;
-    auto kern = a->rounding == LSVD_ROUND_TORCH ? cache_append_wide_kernel<LSVD_ROUND_TORCH>
-                                                : cache_append_wide_kernel<LSVD_ROUND_TRITON>;
-    LSVD_CUDA_TRY(launch_chained(kern, dim3(static_cast<unsigned>(blocks)), dim3(warps_per_block * 32), 0, st, 1, true, p, wt));
+    const size_t smem = static_cast<size_t>(threads) * 2 * sizeof(uint2) + (ahead ? 16 * chunks * 2 * kRowTokens * 2 : 0);
+    // as many blocks as fit an SM (six of 128 threads, by shared memory; else 1024 threads); each walks its share of the tokens
+    const int resident = std::max(1, device_sm_count()) * std::max(1, ahead ? static_cast<int>((220u * 1024u) / (smem + 1024)) : 1024 / threads);
+    void (*kern)(AppendParams, int) =
+        a->rounding == LSVD_ROUND_TORCH ? (ahead ? cache_append_rows_kernel<LSVD_ROUND_TORCH, true> : cache_append_rows_kernel<LSVD_ROUND_TORCH, false>)
+                                        : (ahead ? cache_append_rows_kernel<LSVD_ROUND_TRITON, true> : cache_append_rows_kernel<LSVD_ROUND_TRITON, false>);
+    if (smem > 48 * 1024) LSVD_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), static_cast<int>(smem)));
+    LSVD_CUDA_TRY(launch_chained(kern, dim3(std::min(groups, std::max(1, resident / sides)), sides), dim3(threads), smem, st, 1, true, p,
+                                 (p.side_mask & 1) ? 0 : 1));
     return LSVD_OK;
   }
   const int64_t blocks = (units + warps_per_block - 1) / warps_per_block;

@@ -181,3 +181,38 @@ def test_head_major_layout_holds_the_same_codes(tokens):
     # and the conversion helpers are inverses of each other
     fk, fsk = hm.to_head_major(ck, sk, "k")
     assert torch.equal(fk, hk) and torch.equal(fsk, hsk)
+
+
+@pytest.mark.parametrize("rounding", ["torch", "triton"])
+@pytest.mark.parametrize("head_major", [False, True])
+@pytest.mark.parametrize("pad", [0, 8])
+def test_row_form_equals_the_per_head_form(rounding, head_major, pad):
+    """Every fp16 magnitude, zeros, infinities and NaN through the form for many tokens (four tokens per thread, a remainder
+    of two) and, a few tokens at a time, through the one-warp-per-head form: the same codes and scales, rows at 8-byte
+    alignment included."""
+    k_ranks, v_ranks = [16, 128, 48, 64, 32, 80, 112, 96] * 2, [64, 16, 16, 112, 128, 32, 48, 64] * 2
+    lay = LatentCacheLayout(k_ranks, v_ranks, head_major=head_major)
+    T, N = 2102, 2200
+    gen = torch.Generator().manual_seed(7)
+    bits = torch.randint(0, 0x7bff, (T, lay.sum_k + lay.sum_v), generator=gen).to(torch.int16)
+    both = bits.view(torch.float16) * torch.where(torch.rand(bits.shape, generator=gen) < 0.5, -1, 1).half()
+    both[1::3] = (torch.randn(both[1::3].shape, generator=gen)).half()
+    both[5] = 0
+    both[6, ::40], both[7, 3::50], both[8, 1::30] = float("inf"), float("-inf"), float("nan")
+    both[9, ::2] = float("nan")
+    both = both.cuda()
+    dest = torch.randperm(N, generator=gen)[:T].to(torch.int32).cuda()
+
+    def fresh():
+        if head_major:
+            return [t.zero_() for t in lay.alloc(N)]
+        flat = [torch.zeros(N * (s + pad), dtype=torch.int8, device="cuda") for s in (lay.sum_k, lay.sum_v)]
+        ck, cv = flat[0].view(N, -1)[:, :lay.sum_k], flat[1].view(N, -1)[:, :lay.sum_v]
+        return [ck, torch.zeros(N, 16, dtype=torch.float16, device="cuda"), cv, torch.zeros(N, 16, dtype=torch.float16, device="cuda")]
+
+    many, few = fresh(), fresh()
+    cache_append(lay, both[:, :lay.sum_k], both[:, lay.sum_k:], dest, *many, rounding=rounding)
+    for t in range(0, T, 3):
+        cache_append(lay, both[t:t + 3, :lay.sum_k], both[t:t + 3, lay.sum_k:], dest[t:t + 3].contiguous(), *few, rounding=rounding)
+    for a, b in zip(many, few):
+        assert torch.equal(a.contiguous().view(torch.int8), b.contiguous().view(torch.int8))
