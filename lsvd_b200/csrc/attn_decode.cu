@@ -902,7 +902,7 @@ __global__ void __launch_bounds__(128) merge_up_kernel(const __grid_constant__ M
   // Everything the merge reads is requested at once: the length, the parts' maxima and sums and the first parts' accumulators
   // do not wait for one another.  Parts past the length hold leftovers and are masked.
   // Bound by latency (a few KB a block): with the fixed first items of the stream kernel and the halved up-projection chain below
-  // the whole call goes from 18.8 to 18.4 us (1 x 2048, 32 heads) and from 74.7 to 74.3 us (16 x 4096); 24 x 3001 slot-major: 142, unchanged.
+  // the whole call goes from 18.8 to 18.4 us (1 x 2048, 32 heads) and from 74.7 to 74.3 us (16 x 4096); 24 x 3001 slot-major is unchanged by these.
   const int parts = p.parts[h];
   const float* ml = p.part_ml + (static_cast<int64_t>(b) * p.items_per_request + p.part_off[h]) * 2;
   const int i = threadIdx.x;
