@@ -1,7 +1,8 @@
 // Device functions shared by the stand-alone kernels and the fused decode kernel: the per-token activation
 // quantiser (plain, RMSNorm and sign-FWHT forms), the cache-append rounding, small MMA wrappers.  Each function
 // is the arithmetic of one reference routine; a kernel that calls it produces the same bits whatever launch
-// it sits in.
+// it sits in.  The register-resident quantisers restate it: the block-per-row kernel with the same bits, the
+// warp-per-row kernel of prefills with the RMSNorm's squares added in another order.
 #pragma once
 
 #include "common.cuh"
@@ -99,7 +100,7 @@ struct ActCoder {
   }
 };
 
-// One row by one thread block.  `row`: cols floats of shared memory, `red`: 8 floats.  Every thread of the block
+// One row by one thread block.  `row`: cols floats of shared memory, `red`: 32 floats.  Every thread of the block
 // must call it (block barriers inside); any block size that is a multiple of 32 up to 256.
 __device__ __forceinline__ void act_quant_row(const ActQuantParams& p, int r, float* row, float* red) {
   const __half* x = p.x + r * p.x_row_stride;
@@ -196,14 +197,19 @@ __device__ __forceinline__ void act_quant_row(const ActQuantParams& p, int r, fl
   if (p.norm_weight != nullptr) {
     // RMSNorm as kernels/layer_bench/ffn_kernel/utils.py:560-565: fp32 statistics, the normalised value
     // rounded to fp16, then an fp16 product with the weight.
-    float ss = 0.f;
-    for (int i = threadIdx.x; i < p.cols; i += blockDim.x) ss = fmaf(row[i], row[i], ss);
-    ss = warp_sum(ss);
+    // The squares are added in the order of act_quant_block_kernel, whatever the block size: eight neighbours (and those
+    // 8192 entries on), the 32 sums of a warp of that kernel by shuffles, then its at most 32 warps by shuffles.
+    const int lane = threadIdx.x & 31;
+    const int sums = min(1024, (p.cols + 7) >> 3);
+    for (int c0 = threadIdx.x & ~31; c0 < sums; c0 += blockDim.x) {
+      float ss = 0.f;
+      for (int i0 = (c0 + lane) * 8; i0 < p.cols; i0 += 8192)
+        for (int i = i0; i < min(i0 + 8, p.cols); ++i) ss = fmaf(row[i], row[i], ss);
+      ss = warp_sum(ss);
+      if (lane == 0) red[c0 >> 5] = ss;
+    }
     __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
-    __syncthreads();
-    float tot = 0.f;
-    for (int wi = 0; wi < (blockDim.x >> 5); ++wi) tot += red[wi];
+    const float tot = warp_sum(lane < (sums + 31) >> 5 ? red[lane] : 0.f);
     const float inv = rsqrtf(tot / static_cast<float>(p.cols) + p.norm_eps);
     for (int i = threadIdx.x; i < p.cols; i += blockDim.x) {
       const __half xn = __float2half_rn(row[i] * inv);

@@ -24,7 +24,7 @@ namespace lsvd {
 // ----------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) act_quant_kernel(const __grid_constant__ ActQuantParams p) {
   extern __shared__ float row[];          // cols floats
-  __shared__ float red[8];
+  __shared__ float red[32];
   grid_dependency_wait_release();
   act_quant_row(p, blockIdx.x, row, red);
 }
@@ -117,7 +117,8 @@ __global__ void __launch_bounds__(256, (NCH <= 16 ? 2 : 1)) act_quant_rows_kerne
 // At a few rows the quantiser is a latency: launch, one load, the reductions, one store.  A thread holds NV 16-byte chunks
 // of the row and of the norm weight, all requested at once; each reduction is a warp shuffle, one block barrier and a
 // second shuffle.  act_quant_kernel passes the row through shared memory with scalar loops and five barriers more:
-// RMSNorm + A8 of 16 x 4096 took 11.5 us there.  No rotation, no fp32 input, no fake-quantised output.
+// RMSNorm + A8 of 16 x 4096 took 11.5 us there.  No rotation, no fp32 input, no fake-quantised output.  Same bits as
+// act_quant_row, which adds the RMSNorm's squares in this kernel's order.
 template <int NV>
 __global__ void __launch_bounds__(1024) act_quant_block_kernel(const __grid_constant__ ActQuantParams p) {
   __shared__ float red[2][32];

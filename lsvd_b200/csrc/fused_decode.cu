@@ -733,7 +733,7 @@ fused_decode_kernel(const __grid_constant__ FusedParams p, const __grid_constant
   uint8_t* panel = ring + kFRing;
   uint8_t* scratch = panel + kFPanel;
   __shared__ EngineShared es;
-  __shared__ float red8[8];
+  __shared__ float red8[32];
   __shared__ float zscale[kFMaxTokens * 2];
   __shared__ volatile int aborted;
   __shared__ int flag;

@@ -66,6 +66,19 @@ def test_rmsnorm_rows(rows, cols):
     assert torch.equal(s, s_ref) and torch.equal(q, q_ref)
 
 
+@pytest.mark.parametrize("rows,cols", [(300, 8), (300, 264), (200, 1000), (100, 4096), (60, 5120), (40, 8200), (40, 16384)])
+def test_rmsnorm_of_a_row_does_not_depend_on_its_alignment(rows, cols):
+    """A row at a 2-byte boundary takes the routine that the fused kernel also runs, an aligned one the register-resident
+    kernel: the squares are added in one order, so the statistics, rows, scales and codes are the same bits."""
+    from lsvd_b200.ffn import act_quant
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    x, w = torch.randn(rows, cols, generator=g, device="cuda").half(), (1 + 0.1 * torch.randn(cols, generator=g, device="cuda")).half()
+    odd = torch.empty(rows, cols + 1, dtype=torch.float16, device="cuda")[:, 1:]
+    odd.copy_(x)
+    for a, b in zip(act_quant(x, want_rotated=True, norm_weight=w, norm_eps=1e-5), act_quant(odd, want_rotated=True, norm_weight=w, norm_eps=1e-5)):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("rows", [1, 5, 149, 700])
 @pytest.mark.parametrize("K,nb", [(12, 64), (60, 64), (108, 64), (172, 64), (28, 128), (108, 128), (172, 128)])
 def test_one_token_per_block_rotation(rows, K, nb):
