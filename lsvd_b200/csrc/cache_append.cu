@@ -110,6 +110,81 @@ __global__ void __launch_bounds__(128) cache_append_kernel(const __grid_constant
   if (lane == 0) *scale_unit(p, s, dest, h) = s16;
 }
 
+// Many (token, head) units of few latents a token.  Units are ordered head by head (all tokens of head 0 of K, then head 1,
+// ...), so a warp works on ONE head and its lanes can be dealt by that head's rank: L = 2, 4, 8 or 16 lanes per unit for ranks
+// up to 16, 32, 64, 128, a lane owning 8 consecutive entries (16-byte load, 8-byte store), 32 / L tokens per warp.  The row
+// form below needs a token row that fills a block's lanes: with 1 head of rank 16 (one lane in 32 at work) 131 072 tokens
+// take 61 us there and 7.4 us here, with 8 heads of rank 16 65 536 tokens 33 and 24 us.  Same arithmetic, so the same bits.
+struct WideTable {
+  int32_t warp_begin[2 * LSVD_MAX_HEADS + 1];   // first warp of every (side, head) segment, in launch order
+  int32_t seg_side_head[2 * LSVD_MAX_HEADS];    // side * LSVD_MAX_HEADS + head
+  int32_t nseg;
+};
+
+template <int kRounding>
+__global__ void __launch_bounds__(128) cache_append_wide_kernel(const __grid_constant__ AppendParams p,
+                                                                const __grid_constant__ WideTable w) {
+  grid_dependency_sync();
+  const int lane = threadIdx.x & 31;
+  const int warp_id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (warp_id >= w.warp_begin[w.nseg]) return;
+  int lo_seg = 0, hi_seg = w.nseg;                   // last segment whose first warp is <= warp_id
+  while (hi_seg - lo_seg > 1) {
+    const int mid = (lo_seg + hi_seg) >> 1;
+    if (w.warp_begin[mid] <= warp_id) lo_seg = mid; else hi_seg = mid;
+  }
+  const int side = w.seg_side_head[lo_seg] / LSVD_MAX_HEADS, h = w.seg_side_head[lo_seg] % LSVD_MAX_HEADS;
+  const AppendSide& s = p.side[side];
+  const int r0 = s.rank_off[h];
+  const int rank = s.rank_off[h + 1] - r0;
+  const int lg = rank <= 16 ? 1 : (rank <= 32 ? 2 : (rank <= 64 ? 3 : 4));     // log2 of the lanes per unit
+  const int sub = lane & ((1 << lg) - 1);
+  const int t = (warp_id - w.warp_begin[lo_seg]) * (32 >> lg) + (lane >> lg);
+  const bool live = t < p.num_tokens;
+  const int i0 = sub * 8;
+  const bool active = live && i0 < rank;
+
+  float x[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) x[j] = 0.f;
+  if (active) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(s.latent + static_cast<int64_t>(t) * s.token_stride + s.head_off[h] + i0);
+    const __half2* h2 = reinterpret_cast<const __half2*>(&raw);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      x[2 * j] = __low2float(h2[j]);
+      x[2 * j + 1] = __high2float(h2[j]);
+    }
+  }
+  float amax = 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(x[j]));
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1)
+    if (o < (1 << lg)) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));     // lg is uniform in the warp
+  __half s16 = __float2half_rn(amax * 0.0078125f);
+  const __half floor16 = __float2half_rn(1e-4f);
+  if (__half2float(s16) < __half2float(floor16)) s16 = floor16;
+  const float sf = __half2float(s16);
+  const float rsf = __frcp_rn(sf);
+  if (!live) return;
+  const int dest = p.dest_loc[t];
+  if (dest < 0 || dest >= p.num_slots) {
+    if (sub == 0) report_status(p.status_word, LSVD_ERR_BOUNDS);
+    return;
+  }
+  if (active) {
+    uint32_t lo = 0, hi = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      lo |= (static_cast<uint32_t>(quantise_one<kRounding>(x[j], sf, rsf)) & 0xffu) << (8 * j);
+      hi |= (static_cast<uint32_t>(quantise_one<kRounding>(x[4 + j], sf, rsf)) & 0xffu) << (8 * j);
+    }
+    *reinterpret_cast<uint2*>(cache_unit(p, s, dest, r0, rank) + i0) = make_uint2(lo, hi);
+  }
+  if (sub == 0) *scale_unit(p, s, dest, h) = s16;
+}
+
 // Prefill-sized calls.  A thread owns 16 consecutive latents of one head (a chunk; ranks are multiples of 16) in four tokens
 // at a time and keeps that column for all its tokens, so the head look-up, offsets and strides are paid once per block and a
 // block reads whole token rows: 4 x 32 bytes per thread in flight, contiguous across the block, and one 16-byte store of
@@ -117,8 +192,8 @@ __global__ void __launch_bounds__(128) cache_append_kernel(const __grid_constant
 // barrier per four tokens: the words are double-buffered).  The arithmetic is packed: quotients two at a time in fp32 (as
 // in quantise_one), everything after the rounding to fp16 in fp16 pairs -- adding 1536 rounds to an integer half to even
 // and leaves the code in the low byte -- about seven instructions per latent.
-// 32 768 tokens x (2048 + 2048) latents, 402 MB: 115 us, 3.5 TB/s.  Head-by-head order with eight
-// latents per lane took 224 us (issue bound, and 32..256 bytes of a row at a time).
+// 32 768 tokens x (2048 + 2048) latents, 402 MB: 115 us, 3.5 TB/s.  The head-by-head form above takes 224 us there (issue
+// bound, and 32..256 bytes of a row at a time).
 constexpr int kRowTokens = 4;
 
 // Four codes of (x - already loaded - as two half pairs).  r = 1 / s correctly rounded; a scale that is not finite takes
@@ -285,7 +360,7 @@ __global__ void __launch_bounds__(1024) cache_append_rows_kernel(const __grid_co
   }
 }
 
-// The rows kernel's accesses: 16-byte loads of the latents, stores of at least 8 bytes of the codes.
+// The accesses of the wide and the row form: 16-byte loads of the latents, stores of at least 8 bytes of the codes.
 static bool side_is_wide_ok(const lsvd_append_tensor& t, int num_heads, bool head_major) {
   if (!aligned(t.latent, 16) || (t.token_stride % 8) != 0 || !aligned(t.cache, 8) || (!head_major && (t.cache_row_stride % 8) != 0)) return false;
   for (int h = 0; h < num_heads; ++h) {
@@ -381,17 +456,28 @@ extern "C" int lsvd_cache_append(const lsvd_append_args* a, void* stream) {
   const int64_t units = static_cast<int64_t>(a->num_tokens) * a->num_heads * sides;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int warps_per_block = 4;
-  // One warp per unit up to here: 32 ragged heads, K and V, 64 / 128 / 256 tokens take 2.6 / 3.4 / 5.7 us that way and
-  // 3.1 / 3.2 / 3.3 us in the row form.
-  bool wide = units >= 8192;
-  for (int sd = 0; sd < 2 && wide; ++sd) {
+  bool wide_ok = true;
+  int chunks = 0;                                       // 16-latent chunks of the wider side's token row
+  int64_t latents = 0;
+  for (int sd = 0; sd < 2; ++sd) {
     if (((p.side_mask >> sd) & 1) == 0) continue;
-    wide = side_is_wide_ok(sd == 0 ? a->k : a->v, a->num_heads, p.head_major != 0);
+    const lsvd_append_tensor& t = sd == 0 ? a->k : a->v;
+    wide_ok = wide_ok && side_is_wide_ok(t, a->num_heads, p.head_major != 0);
+    chunks = std::max(chunks, static_cast<int>(t.rank_off[a->num_heads] / 16));
+    latents += static_cast<int64_t>(a->num_tokens) * t.rank_off[a->num_heads];
   }
-  if (wide) {
-    int chunks = 0;
-    for (int sd = 0; sd < 2; ++sd)
-      if ((p.side_mask >> sd) & 1) chunks = std::max(chunks, static_cast<int>((sd == 0 ? a->k : a->v).rank_off[a->num_heads] / 16));
+  // The row form needs rows of at least a warp's chunks (half a warp when there are very many tokens) and enough latents for a
+  // block on most SMs, more the wider the block: a block takes four tokens one after another.  us a call in a row of calls,
+  // K and V, one warp per unit / head by head / rows:
+  //   8 heads of rank 64: 1024 tokens 6.6 / 4.0 / 3.8, 2048 tokens 10.7 / 5.1 / 4.2, 32768 tokens 138 / 45 / 22;
+  //   32 ragged heads, mean 64: 128 tokens 3.5 / 3.6 / 3.2 (alone 8.2 / 8.2 / 10.2), 200 tokens 5.0 / 4.1 / 3.3 (10.3 / 8.7 / 10.3),
+  //     256 tokens 5.8 / - / 3.3;
+  //   128 heads of rank 128: 32 tokens 4.5 / 4.6 / 6.6, 64 tokens 6.6 / 5.9 / 6.5, 128 tokens 10.6 / 8.8 / 6.5;
+  //   16 chunks: 4 heads of rank 64, 4096 tokens 10.6 / 5.0 / 5.3, 16384 tokens 35.7 / 12.4 / 11.5;
+  //   8 chunks: 2 heads of rank 64, 32768 tokens 35.8 / 12.2 / 18.9.
+  const int64_t enough = chunks > 512 ? 4ll << 20 : (chunks > 256 ? 2ll << 20 : 3ll << 18);
+  const bool rows = wide_ok && units >= 12288 && (chunks >= 32 ? latents >= enough : chunks >= 16 && units >= 131072);
+  if (rows) {
     const int threads = (chunks + 31) / 32 * 32;
     const int groups = (a->num_tokens + kRowTokens - 1) / kRowTokens;
     bool ahead = 16 * chunks * 2 * kRowTokens * 2 <= 96 * 1024;
@@ -410,6 +496,31 @@ extern "C" int lsvd_cache_append(const lsvd_append_args* a, void* stream) {
     if (smem > 48 * 1024) LSVD_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), static_cast<int>(smem)));
     LSVD_CUDA_TRY(launch_chained(kern, dim3(std::min(groups, std::max(1, resident / sides)), sides), dim3(threads), smem, st, 1, true, p,
                                  (p.side_mask & 1) ? 0 : 1));
+    return LSVD_OK;
+  }
+  // Head by head above 8192 units (below: 3.2 to 3.6 us either way); few tokens of many heads stay with a warp per unit.
+  if (wide_ok && units > 8192 && a->num_tokens >= 64) {
+    WideTable wt{};
+    int64_t warps = 0;
+    for (int sd = 0; sd < 2; ++sd) {
+      if (((p.side_mask >> sd) & 1) == 0) continue;
+      const lsvd_append_tensor& t = sd == 0 ? a->k : a->v;
+      for (int h = 0; h < a->num_heads; ++h) {
+        const int rank = t.rank_off[h + 1] - t.rank_off[h];
+        const int lanes = rank <= 16 ? 2 : (rank <= 32 ? 4 : (rank <= 64 ? 8 : 16));
+        const int per_warp = 32 / lanes;
+        wt.warp_begin[wt.nseg] = static_cast<int32_t>(warps);
+        wt.seg_side_head[wt.nseg] = sd * LSVD_MAX_HEADS + h;
+        ++wt.nseg;
+        warps += (a->num_tokens + per_warp - 1) / per_warp;
+      }
+    }
+    if (warps > 0x7fffffffLL - 8) return LSVD_ERR_UNSUPPORTED;
+    wt.warp_begin[wt.nseg] = static_cast<int32_t>(warps);
+    const int64_t blocks = (warps + warps_per_block - 1) / warps_per_block;
+    auto kern = a->rounding == LSVD_ROUND_TORCH ? cache_append_wide_kernel<LSVD_ROUND_TORCH>
+                                                : cache_append_wide_kernel<LSVD_ROUND_TRITON>;
+    LSVD_CUDA_TRY(launch_chained(kern, dim3(static_cast<unsigned>(blocks)), dim3(warps_per_block * 32), 0, st, 1, true, p, wt));
     return LSVD_OK;
   }
   const int64_t blocks = (units + warps_per_block - 1) / warps_per_block;

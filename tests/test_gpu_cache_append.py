@@ -158,8 +158,8 @@ def test_append_many_tokens_out_of_range_slots_are_skipped_and_reported():
 @pytest.mark.parametrize("tokens", [37, 2100])
 def test_head_major_layout_holds_the_same_codes(tokens):
     """LSVD_CACHE_HEAD_MAJOR ([H][N_slots][r_h] + scales [H][N_slots]): the same codes and scales as the slot-major
-    cache, in both the decode-sized and the prefill-sized kernel (2100 tokens x 5 heads x 2 sides = 21 000 units < 32 768
-    stays on the first; the second size is reached with 16 heads below)."""
+    cache, in the one-warp-per-unit form (37 tokens x 5 heads x 2 sides) and in the row form (2100 tokens x 16 heads x 2
+    sides of 64 chunks)."""
     gen = torch.Generator().manual_seed(tokens)
     heads = 5 if tokens < 100 else 16
     k_ranks = synth.ragged_ranks(heads, 64, seed=1) if heads == 16 else [16, 128, 48, 64, 32]
@@ -216,3 +216,53 @@ def test_row_form_equals_the_per_head_form(rounding, head_major, pad):
         cache_append(lay, both[t:t + 3, :lay.sum_k], both[t:t + 3, lay.sum_k:], dest[t:t + 3].contiguous(), *few, rounding=rounding)
     for a, b in zip(many, few):
         assert torch.equal(a.contiguous().view(torch.int8), b.contiguous().view(torch.int8))
+
+
+def _same_as_per_head_form(append, tokens, fresh):
+    """``append(slice, caches)`` once for all tokens and a few at a time, through the one-warp-per-head form."""
+    many, few = fresh(), fresh()
+    append(slice(0, tokens), many)
+    for t in range(0, tokens, 3):
+        append(slice(t, t + 3), few)
+    for a, b in zip(many, few):
+        assert torch.equal(a.view(torch.int8), b.view(torch.int8))
+
+
+@pytest.mark.parametrize("rounding", ["torch", "triton"])
+@pytest.mark.parametrize("heads,rank,pad,tokens", [(1, 16, 0, 8195), (1, 128, 8, 8195), (5, 48, 8, 3333), (8, 64, 8, 2051), (32, 64, 16, 515), (64, 128, 0, 259),
+                                                   (128, 128, 8, 259)])
+def test_many_tokens_of_gathered_heads(rounding, heads, rank, pad, tokens):
+    """``destindex_copy_quantize_latent`` on heads that do not lie back to back (or rows too wide for two stages of shared
+    memory), from one 16-latent chunk a token to a block of 1024 threads: the head-by-head form below 16 chunks, register loads
+    of the row form above."""
+    gen = torch.Generator().manual_seed(heads + rank)
+    lat = torch.randn(tokens, heads, rank + pad, generator=gen).half().cuda()[:, :, :rank]
+    lat[5], lat[6, 0, 3], lat[7, -1, -1] = 0, float("inf"), float("nan")
+    dest = torch.randperm(tokens + 40, generator=gen)[:tokens].int().cuda()
+
+    def append(s, caches):
+        destindex_copy_quantize_latent(lat[s], dest[s], *caches, rounding=rounding)
+    _same_as_per_head_form(append, tokens, lambda: (torch.zeros(tokens + 40, heads, rank, dtype=torch.int8, device="cuda"),
+                                                    torch.zeros(tokens + 40, heads, dtype=torch.float16, device="cuda")))
+
+
+@pytest.mark.parametrize("head_major", [False, True])
+@pytest.mark.parametrize("heads,rank,tokens", [(1, 16, 4097), (2, 64, 2050), (8, 16, 515), (8, 32, 9001), (4, 128, 2051), (32, 64, 130), (32, 64, 194), (64, 128, 131), (128, 128, 33),
+                                               (128, 128, 66), (128, 128, 130)])
+def test_every_form_of_the_append_writes_the_same(head_major, heads, rank, tokens):
+    """Both sides of the lines between the forms: rows of 1 to 1024 chunks, a remainder of tokens, both cache layouts, slots
+    out of range (skipped and reported)."""
+    lay = LatentCacheLayout.uniform(heads, rank)
+    lay = lay.as_head_major() if head_major else lay
+    gen = torch.Generator().manual_seed(heads + rank)
+    both = torch.randn(tokens, 2, lay.sum_k, generator=gen).half().cuda()
+    both[3] = 0
+    dest = torch.randperm(tokens + 40, generator=gen)[:tokens].int().cuda()
+    dest[1], dest[tokens - 1] = -1, tokens + 40
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    cache_append(lay, both[:, 0], both[:, 1], dest, *[t.zero_() for t in lay.alloc(tokens + 40)], status_word=status)
+    assert int(status) == 6
+
+    def append(s, caches):
+        cache_append(lay, both[s, 0], both[s, 1], dest[s], *caches)
+    _same_as_per_head_form(append, tokens, lambda: [t.zero_() for t in lay.alloc(tokens + 40)])
