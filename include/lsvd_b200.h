@@ -338,7 +338,7 @@ int lsvd_heads_hadamard_partial(const void* x, int64_t x_row_stride, const int32
  *   epilogue 0: out[m, out_col + n] = fp16((acc * a_scale[m]) * w_scale[n])              (a quantised Linear)
  *   epilogue 1: g = that for (w, a), u = that for (w2, a2); out = fp16(fp16(silu(g)) * u) (gate/up pair)
  *   epilogue 2: the same pair with g, u kept in fp32: out = fp16(u * (g * sigmoid(g))), the convention of
- *               kernels/layer_bench/ffn_kernel/mix_ffn_kernel.py:353-362,1885-1889 (forms 0 and 3 only)
+ *               kernels/layer_bench/ffn_kernel/mix_ffn_kernel.py:353-362,1885-1889 (not forms 1 and 2)
  * With row_absmax the call also folds max |fp32 value before the fp16 rounding| of every token into a device
  * word per token (atomic maximum on the float's bit pattern; the caller zeroes it), which is what the reference's
  * tiled kernels hand to their next quantiser (mix_ffn_kernel.py:1229-1232, 1894-1895).
@@ -361,20 +361,22 @@ typedef struct lsvd_gemv_args {
   int64_t residual_row_stride;
   int32_t* status_word;          /* device int32 or NULL: LSVD_ERR_TIMEOUT if a pipeline wait of the   */
                                  /* TMA-fed form ran out; the output is then incomplete               */
-  int32_t form;                  /* 0: tcgen05 kernel, every size;                                        */
+  int32_t form;                  /* 0: chosen by size (and by prefetch_weights: below);                   */
                                  /* 1: persistent TMA-fed kernel with K split over warps, m <= 16 only   */
                                  /*    (LSVD_ERR_UNSUPPORTED beyond); 2: TMA-fed kernel whose warps      */
                                  /*    share the token rows (built for 17..64 tokens, valid for any m);   */
-                                 /* 3: register-fed kernel for any m.  Same values in every form.        */
-  uint32_t* row_absmax;          /* optional device words [m * row_absmax_stride]: see above (forms 0, 3)  */
+                                 /* 3: register-fed kernel for any m; 4: tcgen05 kernel for any m.       */
+                                 /* Same values in every form.                                           */
+  uint32_t* row_absmax;          /* optional device words [m * row_absmax_stride]: see above (not forms 1, 2) */
   int64_t row_absmax_stride;     /* words between two tokens                                              */
   int32_t absmax_split;          /* 0: one word per token; else channels >= absmax_split (a multiple of  */
                                  /* 16) go to the token's second word                                     */
-  int32_t prefetch_weights;      /* every block asks for its weights (form 0: the first stages of its ring, form 3: */
+  int32_t prefetch_weights;      /* every block asks for its weights (form 4: the first stages of its ring, form 3: */
                                  /* L2 prefetch) before it waits for the kernel launched before it on the stream.    */
                                  /* Set it only behind one of this library's kernels: the weights must be complete   */
-                                 /* when that kernel starts.  Results do not depend on it.                           */
-  float* out_f32;                /* optional device fp32 [m, n] (single product, forms 0 and 3): (acc * a_scale) * w_scale  */
+                                 /* when that kernel starts.  Form 0 then is the tcgen05 kernel.  Results do not     */
+                                 /* depend on it.                                                                    */
+  float* out_f32;                /* optional device fp32 [m, n] (single product, not forms 1 and 2): (acc * a_scale) * w_scale */
                                  /* with no fp16 rounding -- the partial sum a row-parallel rank sends to the all-reduce  */
 } lsvd_gemv_args;
 int lsvd_w8a8_gemv(const lsvd_gemv_args* args, void* stream);

@@ -937,6 +937,27 @@ extern "C" int lsvd_hadamard_quant(const lsvd_hadamard_quant_args* a, void* stre
   return LSVD_OK;
 }
 
+namespace lsvd {
+// Form 0: the tcgen05 kernel or the register-fed one.  Behind a quantiser that lets it ask for its weights early the tcgen05
+// kernel is the faster one at every size (figures in gemv_tc.cu).  A product on its own pays for the cluster's start and for
+// the sums across it; us a call with weights from HBM, register-fed / tcgen05:
+//   1 token: 4096 x 4096 12.3 / 14.4, 5504 x 512 pair 10.3 / 12.3, 5504 x 4096 pair 18.5 / 21.7, 32000 x 4096 36.9 / 39.0;
+//            but 4096 x 11008 24.5 / 20.5 and 256 x 14336 22.6 / 14.4 (a long K in 16 channels a block);
+//   16 tokens: 5504 x 4096 pair 20.5 / 24.6, 12288 x 4096 22.6 / 22.6, 32000 x 256 14.4 / 12.3, 32000 x 4096 43.0 / 39.5;
+//   32 tokens: 1024 x 512 8.2 / 10.3, 4096 x 4096 14.5 / 15.3, 5504 x 4096 pair 26.7 / 24.6, 12288 x 4096 25.8 / 22.5,
+//              16384 x 16 12.3 / 10.6;
+//   64 tokens: 1024 x 512 10.3 / 10.3, 4096 x 512 10.3 / 11.4, 1024 x 1024 pair 18.4 / 14.4, 5504 x 512 pair 20.5 / 16.4;
+//              4 MB and more 16.4 / 12.4 to 75.9 / 41.0 (the shared-token form, which took these before).
+static bool tc_is_faster(const lsvd_gemv_args* a, bool dual) {
+  if (a->prefetch_weights != 0) return true;
+  const int64_t bytes = static_cast<int64_t>(a->n) * a->k * (dual ? 2 : 1);
+  if (a->k >= 8192) return true;
+  if (!dual && a->n >= 16384 && (a->m > 16 || (a->m > 8 && a->k >= 256))) return true;
+  if (a->m > 32) return bytes >= (dual ? 2ll : 4ll) << 20;
+  return a->m > 16 && bytes >= 32ll << 20;
+}
+}  // namespace lsvd
+
 extern "C" int lsvd_w8a8_gemv(const lsvd_gemv_args* a, void* stream) {
   using namespace lsvd;
   if (a == nullptr || a->m <= 0 || a->m > 64 || a->n <= 0 || (a->n % 16) || a->k <= 0 || (a->k % 16))
@@ -945,7 +966,7 @@ extern "C" int lsvd_w8a8_gemv(const lsvd_gemv_args* a, void* stream) {
   if ((a->out != nullptr || a->out_f32 != nullptr) && (!a->w_scale || !a->a_scale)) return LSVD_ERR_INVALID_ARG;
   const bool dual = a->w2 != nullptr;
   if (dual != (a->epilogue == 1 || a->epilogue == 2) || a->epilogue < 0 || a->epilogue > 2) return LSVD_ERR_INVALID_ARG;
-  const bool fp32_form = a->epilogue == 2 || a->row_absmax != nullptr;     // built into the register-fed kernel only
+  const bool fp32_form = a->epilogue == 2 || a->row_absmax != nullptr;     // not built into forms 1 and 2
   if (fp32_form && (a->form == 1 || a->form == 2)) return LSVD_ERR_UNSUPPORTED;
   if (a->row_absmax != nullptr && (a->out == nullptr || a->absmax_split < 0 || (a->absmax_split % 16))) return LSVD_ERR_INVALID_ARG;
   if (dual && a->out != nullptr && !a->w2_scale) return LSVD_ERR_INVALID_ARG;
@@ -972,11 +993,8 @@ extern "C" int lsvd_w8a8_gemv(const lsvd_gemv_args* a, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (a->form == 1) return a->m <= 16 ? launch_gemv_streamed(p, dual, split, st) : LSVD_ERR_UNSUPPORTED;
   if (a->form == 2) return launch_gemv_wide(p, dual, split, st);
-  if (a->form != 0 && a->form != 3) return LSVD_ERR_INVALID_ARG;
-  // Form 0 at every size: at 1 token the tcgen05 form and the register-fed one are level on the 4 MB product (the chain's
-  // other kernels bound it) and 45 MB take 15 instead of 17 us with their quantiser; from 17 tokens on it is 1.3 to 3
-  // times as fast (figures in gemv_tc.cu).
-  if (a->form == 0) return launch_gemv_tc(p, dual, split, st);
+  if (a->form < 0 || a->form > 4) return LSVD_ERR_INVALID_ARG;
+  if (a->form == 4 || (a->form == 0 && tc_is_faster(a, dual))) return launch_gemv_tc(p, dual, split, st);
   if (a->m <= 8) return launch_gemv_nt<1>(p, dual, split, st);
   if (a->m <= 16) return launch_gemv_nt<2>(p, dual, split, st);
   if (a->m <= 32) return launch_gemv_nt<4>(p, dual, split, st);

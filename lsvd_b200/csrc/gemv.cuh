@@ -26,7 +26,7 @@ struct GemvParams {
 int launch_gemv_streamed(const GemvParams& p, bool dual, bool split, cudaStream_t st);
 // The TMA-fed form for 17..64 tokens: token rows shared by the block's warps through shared memory.
 int launch_gemv_wide(const GemvParams& p, bool dual, bool split, cudaStream_t st);
-// The tcgen05 form (gemv_tc.cu), the default for 1..64 tokens.
+// The tcgen05 form (gemv_tc.cu), for 1..64 tokens.
 int launch_gemv_tc(const GemvParams& p, bool dual, bool split, cudaStream_t st);
 
 #ifdef __CUDACC__

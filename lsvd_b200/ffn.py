@@ -172,8 +172,8 @@ def w8a8_gemv(a_q, a_scale, w_q, w_scale, w2_q=None, w2_scale=None, a2_q=None, a
               row_absmax=None, absmax_split=0, prefetch_weights=False, out_f32=None, acc=None):
     """acc = a_q @ w_q^T (int32, exact) for 1..64 tokens, dequantised to fp16; with (w2, a2) a gate/up pair whose
     result is silu(gate) * up.  Returns (out fp16 [m, n] or the passed tensor, acc int32 or None, acc2 or None).
-    ``form`` 0 is the tcgen05 kernel, 1 the persistent TMA-fed one (at most 16 tokens), 2 the wide one, 3 the
-    register-fed one; ``status_word`` (int32 device tensor) receives LSVD_ERR_TIMEOUT if a pipeline wait gives up.  ``fp32_swiglu`` selects the
+    ``form`` 0 is chosen by size, 1 the persistent TMA-fed kernel (at most 16 tokens), 2 the wide one, 3 the
+    register-fed one, 4 the tcgen05 one; ``status_word`` (int32 device tensor) receives LSVD_ERR_TIMEOUT if a pipeline wait gives up.  ``fp32_swiglu`` selects the
     all-fp32 gate/up epilogue ``up * (gate * sigmoid(gate))``; ``row_absmax`` (int32 view of the words, strided by
     token) collects max |fp32 value| per token, channels from ``absmax_split`` on in the token's second word."""
     _require_cuda(a_q, w_q)

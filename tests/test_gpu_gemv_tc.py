@@ -1,4 +1,4 @@
-"""The default (tcgen05) form of the weight-streaming product: tile edges, remainders of K and tokens, every epilogue."""
+"""The tcgen05 form of the weight-streaming product: tile edges, remainders of K and tokens, every epilogue."""
 import pytest
 import torch
 
@@ -37,7 +37,7 @@ def test_accumulators_and_results(m, n, k, kind):
     res = torch.randn(m, n + 3, device="cuda").half()[:, 1:n + 1] if not dual else None      # odd stride, 2-byte aligned
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     buf = [torch.zeros(m, n + 5, dtype=torch.float16, device="cuda") for _ in range(2)]
-    got = w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], want_acc=True, residual=res, out=buf[0], out_col=3, status_word=status, **kw)
+    got = w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], want_acc=True, residual=res, out=buf[0], out_col=3, status_word=status, form=4, **kw)
     want = w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], want_acc=True, residual=res, out=buf[1], out_col=3, form=3, **kw)
     assert int(status) == 0
     exact = d["a"].double() @ d["w"].double().t()
@@ -48,11 +48,27 @@ def test_accumulators_and_results(m, n, k, kind):
     assert torch.equal(buf[0], buf[1])                                     # untouched border columns included
     if not dual:
         o32 = [torch.empty(m, n, device="cuda") for _ in range(2)]
-        w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], want_out=False, out_f32=o32[0])
+        w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], want_out=False, out_f32=o32[0], form=4)
         w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], want_out=False, out_f32=o32[1], form=3)
         assert torch.equal(o32[0], o32[1])
     words = [torch.zeros(m, 4, dtype=torch.int32, device="cuda") for _ in range(2)]
     outs = [w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], fp32_swiglu=dual, row_absmax=words[i], absmax_split=16 if n > 16 else 0,
-                      form=3 * i, prefetch_weights=i == 0, **kw)[0] for i in range(2)]
+                      form=4 - i, prefetch_weights=i == 0, **kw)[0] for i in range(2)]
     assert torch.equal(outs[0], outs[1])
     assert torch.equal(words[0], words[1])
+
+
+@pytest.mark.parametrize("m,n,k,dual", [(1, 4096, 512, False), (8, 256, 8192, False), (8, 256, 8176, False), (9, 16384, 256, False), (9, 16368, 256, False),
+                                        (17, 16384, 16, False), (17, 8192, 4096, False), (16, 8192, 4096, False), (33, 1024, 4096, False), (33, 1008, 4096, False), (33, 1024, 1024, True),
+                                        (33, 1008, 1024, True)])
+def test_the_form_chosen_by_size_has_the_same_bits(m, n, k, dual):
+    """Both sides of each line of the choice, with and without an early request for the weights."""
+    from lsvd_b200.ffn import w8a8_gemv
+    d = _case(m, n, k, dual, False, seed=n)
+    kw = dict(w2_q=d["w2"], w2_scale=d["ws2"]) if dual else {}
+    want = w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], want_acc=True, form=3, **kw)
+    torch.cuda.synchronize()
+    for early in (False, True):
+        got = w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], want_acc=True, prefetch_weights=early, **kw)
+        for x, y in zip(got, want):
+            assert x is y is None or torch.equal(x, y)
