@@ -469,13 +469,17 @@ __global__ void __launch_bounds__(kStreamThreads, 1) latent_stream_kernel(const 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   grid_dependency_sync();
 
-  // Items: (request b, head h, part k).  A warp's first one is fixed, which spares the launch a round trip to the counter.
-  if (lane == 0) first_item[warp] = blockIdx.x * kStreamWarps + warp;
+  // Items: (request b, head h, part k).  When every item finds a warp, warp w of block b takes item w * blocks + b: no round
+  // trip to the counter, and the parts of a head of large rank lie on different SMs (block by block, 1 x 1024 with ragged
+  // ranks used 43 of 64 blocks: 18.2 us a call against 14.8).  Otherwise all items come from the counter.  The item passes
+  // through shared memory so that the compiler keeps one copy of the loop's body (two: 10 to 25 % slower).
+  const int fixed = p.total_items <= static_cast<int>(gridDim.x) * kStreamWarps ? static_cast<int>(gridDim.x) * kStreamWarps : 0;
+  if (lane == 0) first_item[warp] = fixed > 0 ? warp * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x) : -1;
   for (;;) {
     int item = 0;
     if (lane == 0) {
       item = first_item[warp];
-      if (item < 0) item = atomicAdd(p.queue, 1) + gridDim.x * kStreamWarps;
+      if (item < 0) item = atomicAdd(p.queue, 1) + fixed;
       first_item[warp] = -1;
     }
     item = __shfl_sync(0xffffffffu, item, 0);
@@ -828,13 +832,14 @@ __global__ void __launch_bounds__(kRingThreads, 1) latent_stream_ring_kernel(con
   grid_dependency_sync();
   uint32_t phases = 0u;              // bit s: the parity of stage s's next completion
 
-  // Items: (request b, head h, part k).  A warp's first one is fixed, which spares the launch a round trip to the counter.
-  if (lane == 0) first_item[warp] = blockIdx.x * kRingWarps + warp;
+  // Items as in latent_stream_kernel.
+  const int fixed = p.total_items <= static_cast<int>(gridDim.x) * kRingWarps ? static_cast<int>(gridDim.x) * kRingWarps : 0;
+  if (lane == 0) first_item[warp] = fixed > 0 ? warp * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x) : -1;
   for (;;) {
     int item = 0;
     if (lane == 0) {
       item = first_item[warp];
-      if (item < 0) item = atomicAdd(p.queue, 1) + gridDim.x * kRingWarps;
+      if (item < 0) item = atomicAdd(p.queue, 1) + fixed;
       first_item[warp] = -1;
     }
     item = __shfl_sync(0xffffffffu, item, 0);
@@ -901,8 +906,8 @@ __global__ void __launch_bounds__(128) merge_up_kernel(const __grid_constant__ M
   grid_dependency_wait();
   // Everything the merge reads is requested at once: the length, the parts' maxima and sums and the first parts' accumulators
   // do not wait for one another.  Parts past the length hold leftovers and are masked.
-  // Bound by latency (a few KB a block): with the fixed first items of the stream kernel and the halved up-projection chain below
-  // the whole call goes from 18.8 to 18.4 us (1 x 2048, 32 heads) and from 74.7 to 74.3 us (16 x 4096); 24 x 3001 slot-major is unchanged by these.
+  // Bound by latency (a few KB a block).  Together with the fixed items of the stream kernel a call takes 13.9 instead of 16.1 us
+  // at 1 x 200 and 14.9 instead of 16.2 at 1 x 1024 (32 ragged heads, head-major); from 8 x 1000 on nothing changes.
   const int parts = p.parts[h];
   const float* ml = p.part_ml + (static_cast<int64_t>(b) * p.items_per_request + p.part_off[h]) * 2;
   const int i = threadIdx.x;
@@ -1221,12 +1226,17 @@ int attn_launch_stream(const lsvd_attn_decode_args* a, const AttnLaunch& L, cuda
     return e != nullptr && std::atoi(e) == 2;
   }();
   const int ring_smem = kRingWarps * kRingBytesPerWarp;
+  // A block of the ring form fills an SM's shared memory.  While the items fit into the warps of eight blocks fewer, those SMs
+  // stay free for the merge's blocks, which start early and fetch the V up-factor while the cache is read: 4 x 800 alone
+  // 32.8 us with every SM taken, 27.3 so; 1 x 3000 34.8 and 28.6.
+  const int64_t most = std::max(1, device_sm_count() - 8);
+  const int ring_blocks = hp.total_items <= most * kRingWarps ? static_cast<int>(std::min<int64_t>(hp.num_blocks, most)) : hp.num_blocks;
   if (use_ring && sp.head_major) {
     LSVD_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(latent_stream_ring_kernel<true>), ring_smem));
-    LSVD_CUDA_TRY(launch_chained(latent_stream_ring_kernel<true>, dim3(hp.num_blocks), dim3(kRingThreads), ring_smem, st, 1, true, sp));
+    LSVD_CUDA_TRY(launch_chained(latent_stream_ring_kernel<true>, dim3(ring_blocks), dim3(kRingThreads), ring_smem, st, 1, true, sp));
   } else if (ring_slot_major && !sp.head_major) {
     LSVD_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(latent_stream_ring_kernel<false>), ring_smem));
-    LSVD_CUDA_TRY(launch_chained(latent_stream_ring_kernel<false>, dim3(hp.num_blocks), dim3(kRingThreads), ring_smem, st, 1, true, sp));
+    LSVD_CUDA_TRY(launch_chained(latent_stream_ring_kernel<false>, dim3(ring_blocks), dim3(kRingThreads), ring_smem, st, 1, true, sp));
   } else if (sp.head_major) LSVD_CUDA_TRY(launch_chained(latent_stream_kernel<true>, dim3(hp.num_blocks), dim3(kStreamThreads), 0, st, 1, true, sp));
   else LSVD_CUDA_TRY(launch_chained(latent_stream_kernel<false>, dim3(hp.num_blocks), dim3(kStreamThreads), 0, st, 1, true, sp));
   if (a->ev_stream_end) LSVD_CUDA_TRY(cudaEventRecord(static_cast<cudaEvent_t>(a->ev_stream_end), st));

@@ -228,3 +228,19 @@ def test_bad_request_row_and_overlong_length_are_reported():
     assert status.item() == 6 and torch.equal(o[0], good[0]) and (o[1] == 0).all()
     o = run(lambda st: st.b_seq_len.copy_(torch.tensor([64, 1000], dtype=torch.int32)))      # max_len_in_batch stays 64
     assert status.item() == 6 and torch.isfinite(o.float()).all() and torch.equal(o[0], good[0])
+
+
+@pytest.mark.parametrize("warps", [lambda s: 16 * s, lambda s: 24 * (s - 8), lambda s: 24 * s])
+@pytest.mark.parametrize("more", [0, 32])
+def test_as_many_items_as_warps_and_one_round_more(warps, more):
+    """Items of one tile (32 tokens of a head): exactly as many as a grid of the register-fed (16 warps an SM) or of the ring
+    form (24, eight SMs left free or all taken) has warps, and 32 more -- the fixed items and the counter, in both layouts."""
+    import ctypes as C
+    from lsvd_b200 import _lib
+    L = warps(torch.cuda.get_device_properties(0).multi_processor_count) + more
+    c = U.build_case(1, 32, 128, [64] * 32, [64] * 32, [L], seed=L)
+    off = _lib.i32_array(c["k_off"])
+    items = C.c_int32()
+    _lib.check(_lib.load().lsvd_attn_decode_plan(1, 32, off, off, L, C.byref(items), None, None))
+    assert items.value == L
+    assert torch.equal(check(c), U.run_gpu(c, head_major=True))
