@@ -1237,8 +1237,16 @@ int attn_launch_stream(const lsvd_attn_decode_args* a, const AttnLaunch& L, cuda
   } else if (ring_slot_major && !sp.head_major) {
     LSVD_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(latent_stream_ring_kernel<false>), ring_smem));
     LSVD_CUDA_TRY(launch_chained(latent_stream_ring_kernel<false>, dim3(ring_blocks), dim3(kRingThreads), ring_smem, st, 1, true, sp));
-  } else if (sp.head_major) LSVD_CUDA_TRY(launch_chained(latent_stream_kernel<true>, dim3(hp.num_blocks), dim3(kStreamThreads), 0, st, 1, true, sp));
-  else LSVD_CUDA_TRY(launch_chained(latent_stream_kernel<false>, dim3(hp.num_blocks), dim3(kStreamThreads), 0, st, 1, true, sp));
+  } else {
+    // The register-fed form lives on L1: a step's rows come in pieces of 16 bytes of the same lines.  Its blocks stay for the
+    // whole stream, and the split of an SM between L1 and shared memory stays the one that its first block found there:
+    // behind a product (two blocks of 110 KB) or a merge (16 KB a block), launched programmatically, a few KB of L1.  The
+    // preference below makes the launch wait for the split it needs instead.  us: 24 x 3001 shuffled slots, calls in a
+    // row 166 without, 101 with it; a decoder layer of 16 x 4096 on the slot-major layout 190 and 149, of 6 x 3001 126 and 102.
+    void (*kern)(StreamParams) = sp.head_major ? latent_stream_kernel<true> : latent_stream_kernel<false>;
+    LSVD_CUDA_TRY(ensure_large_l1(reinterpret_cast<const void*>(kern)));
+    LSVD_CUDA_TRY(launch_chained(kern, dim3(hp.num_blocks), dim3(kStreamThreads), 0, st, 1, true, sp));
+  }
   if (a->ev_stream_end) LSVD_CUDA_TRY(cudaEventRecord(static_cast<cudaEvent_t>(a->ev_stream_end), st));
   return LSVD_OK;
 }

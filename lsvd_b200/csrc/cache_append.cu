@@ -526,14 +526,9 @@ extern "C" int lsvd_cache_append(const lsvd_append_args* a, void* stream) {
   const int64_t blocks = (units + warps_per_block - 1) / warps_per_block;
   if (blocks > 0x7fffffffLL) return LSVD_ERR_UNSUPPORTED;
   const dim3 grid(static_cast<unsigned>(blocks)), block(warps_per_block * 32);
-  // On the slot-major layout a large batch's append starts a plain launch: chained, decode calls that follow one another overlap
-  // and disturb the scattered reads of the register-fed stream (24 x 3001 tokens, 1536 units: 142 us a call chained, 88 us plain).
-  // Small batches gain from the early start (1 x 2048, 64 units: 18.5 chained, 19.2 plain), and so does the head-major layout
-  // (16 x 4096: 65 against 74 us in a row of calls).
-  const bool chained = p.head_major || units < 512;
   if (a->rounding == LSVD_ROUND_TORCH)
-    LSVD_CUDA_TRY(launch_chained(cache_append_kernel<LSVD_ROUND_TORCH>, grid, block, 0, st, 1, chained, p));
+    LSVD_CUDA_TRY(launch_chained(cache_append_kernel<LSVD_ROUND_TORCH>, grid, block, 0, st, 1, true, p));
   else
-    LSVD_CUDA_TRY(launch_chained(cache_append_kernel<LSVD_ROUND_TRITON>, grid, block, 0, st, 1, chained, p));
+    LSVD_CUDA_TRY(launch_chained(cache_append_kernel<LSVD_ROUND_TRITON>, grid, block, 0, st, 1, true, p));
   return LSVD_OK;
 }

@@ -2,6 +2,7 @@
 #include <cstdlib>
 #include <map>
 #include <mutex>
+#include <set>
 #include <utility>
 
 #include "common.cuh"
@@ -20,6 +21,7 @@ struct DeviceInfo {
 static std::mutex g_mu;
 static std::map<int, DeviceInfo> g_devices;
 static std::map<std::pair<int, const void*>, int> g_smem_set;
+static std::set<std::pair<int, const void*>> g_large_l1;
 
 static const DeviceInfo* current_device_info() {
   int dev = 0;
@@ -69,6 +71,17 @@ cudaError_t ensure_dynamic_smem(const void* kernel, int bytes) {
   if (have >= bytes) return cudaSuccess;
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e == cudaSuccess) have = bytes;
+  return e;
+}
+
+cudaError_t ensure_large_l1(const void* kernel) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(g_mu);
+  if (g_large_l1.count({dev, kernel}) != 0) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
+  if (e == cudaSuccess) g_large_l1.insert({dev, kernel});
   return e;
 }
 

@@ -30,6 +30,8 @@ int device_sm_count();           // SM count of the current device (cached per d
 int device_max_smem_optin();     // opt-in shared memory per block of the current device
 // Raise a kernel's dynamic shared memory limit on the current device (remembered, so repeated calls are free).
 cudaError_t ensure_dynamic_smem(const void* kernel, int bytes);
+// Ask for the largest L1 that the kernel's static shared memory leaves on the current device (remembered as well).
+cudaError_t ensure_large_l1(const void* kernel);
 
 // Kernels of one decode step run back to back on a stream, each a few microseconds long.  They are launched
 // with programmatic stream serialisation: the next kernel's blocks may become resident while the previous
