@@ -185,28 +185,37 @@ __global__ void __launch_bounds__(KT * 32, PER_SM) hadamard_tokens_kernel(const 
   }
 }
 
-template <int KT, int NB>
+template <int KT, int NB, int PER_SM>
 static int launch_tokens(const HadQuantParams& p, cudaStream_t st) {
   const int smem = 3 * p.Kp * (NB + 8) * 2;
   const int sms = std::max(1, device_sm_count());
-  // a token per SM at most: all the registers a block can use (the two-per-SM budget spills at K = 172)
-  void (*kern)(HadQuantParams) = p.rows <= sms ? hadamard_tokens_kernel<KT, NB, 1> : hadamard_tokens_kernel<KT, NB, 2>;
+  void (*kern)(HadQuantParams) = hadamard_tokens_kernel<KT, NB, PER_SM>;
   if (smem > 48 * 1024) LSVD_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
-  LSVD_CUDA_TRY(launch_chained(kern, dim3(std::min(p.rows, 2 * sms)), dim3(KT * 32), smem, st, 1, true, p));
+  LSVD_CUDA_TRY(launch_chained(kern, dim3(std::min(p.rows, PER_SM * sms)), dim3(KT * 32), smem, st, 1, true, p));
   return LSVD_OK;
 }
 
+// Blocks per SM.  A token per SM at most gets all the registers a block can use.  More tokens get as many blocks as shared
+// memory and about 128 registers a thread admit: two of 11 warps at nb = 64 (80 registers, some spills, and still faster:
+// 8191 tokens of 172 x 64 226 against 273 us), but one at 172 x 128, whose 144 KB fit once (built for two, 80 registers and
+// 184 bytes of spills: 8000 tokens 555 us, so 369).  had_K of one or two tiles takes a block of as many warps, and many
+// blocks: 8000 tokens of 12 x 64 took 45 us with four warps, three of them without a tile, and take 11.4; 28 x 64 52 and 20.5.
 int launch_hadamard_tokens(const HadQuantParams& p, cudaStream_t st) {
   if ((p.nb != 64 && p.nb != 128) || p.Kp > 176 || !p.x_vec16) return LSVD_ERR_UNSUPPORTED;
   const int tiles = p.Kp >> 4;
+  const bool many = p.rows > device_sm_count();
   if (p.nb == 64) {
-    if (tiles <= 4) return launch_tokens<4, 64>(p, st);
-    if (tiles <= 7) return launch_tokens<7, 64>(p, st);
-    return launch_tokens<11, 64>(p, st);
+    if (many && tiles == 1) return launch_tokens<1, 64, 16>(p, st);
+    if (many && tiles == 2) return launch_tokens<2, 64, 8>(p, st);
+    if (tiles <= 4) return many ? launch_tokens<4, 64, 2>(p, st) : launch_tokens<4, 64, 1>(p, st);
+    if (tiles <= 7) return many ? launch_tokens<7, 64, 2>(p, st) : launch_tokens<7, 64, 1>(p, st);
+    return many ? launch_tokens<11, 64, 2>(p, st) : launch_tokens<11, 64, 1>(p, st);
   }
-  if (tiles <= 4) return launch_tokens<4, 128>(p, st);
-  if (tiles <= 7) return launch_tokens<7, 128>(p, st);
-  return launch_tokens<11, 128>(p, st);
+  if (many && tiles == 1) return launch_tokens<1, 128, 16>(p, st);
+  if (many && tiles == 2) return launch_tokens<2, 128, 8>(p, st);
+  if (tiles <= 4) return many ? launch_tokens<4, 128, 2>(p, st) : launch_tokens<4, 128, 1>(p, st);
+  if (tiles <= 7) return many ? launch_tokens<7, 128, 2>(p, st) : launch_tokens<7, 128, 1>(p, st);
+  return launch_tokens<11, 128, 1>(p, st);
 }
 
 }  // namespace lsvd

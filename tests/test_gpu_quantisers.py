@@ -79,8 +79,9 @@ def test_rmsnorm_of_a_row_does_not_depend_on_its_alignment(rows, cols):
         assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("rows", [1, 5, 149, 700])
-@pytest.mark.parametrize("K,nb", [(12, 64), (60, 64), (108, 64), (172, 64), (28, 128), (108, 128), (172, 128)])
+@pytest.mark.parametrize("rows", [1, 5, 149, 700, 2500])
+@pytest.mark.parametrize("K,nb", [(12, 64), (16, 64), (28, 64), (32, 64), (60, 64), (108, 64), (172, 64), (12, 128), (28, 128), (60, 128), (108, 128),
+                                  (172, 128)])
 def test_one_token_per_block_rotation(rows, K, nb):
     """Against the oracle's rotation on the CPU: had_K is +-1 and the sums of up to 172 fp16 values are taken in fp32 in another
     order, so a result may round the other way (one fp16 step); codes and scale follow from the rotated row exactly.  The
