@@ -17,8 +17,8 @@
 // from HBM): the stream itself runs at 6 TB/s; a block spends about 1 us on its start and 1.5 to 3 us on the sums and the
 // epilogue.  Hybrid FFN 4096/11008 at 1 / 29 tokens 51.3 / 62.2 -> 45.3 / 55.5 us per call, 5120/13824 at 64 tokens
 // 159 -> 88 us, mixffn 4096/14336 at 32 tokens 124 -> 79 us.
-// Every wait on an mbarrier is bounded; one that gives up reports LSVD_ERR_TIMEOUT, and the block still attends the
-// cluster barriers, waits for its own copies and releases its tensor memory.
+// Every wait on an mbarrier is bounded; one that gives up, in whatever role, reports LSVD_ERR_TIMEOUT, and the block still
+// attends the cluster barriers, waits for its own copies and MMAs and releases its tensor memory.
 #include <algorithm>
 
 #include "gemv.cuh"
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) w8a8_gemv_tc_kernel(const __gri
   const int tile = blockIdx.x >> CSL;
   const int nb = p.split ? 2 * p.ntok : p.ntok;                    // columns of the MMA
   const int stage_bytes = kTcWBytes + nb * 128;
-  const int nk = p.kb > rank ? (p.kb - rank + cs - 1) >> CSL : 0;  // this block's K blocks: rank, rank + cs, ...
+  const int nk = (p.kb - rank + cs - 1) >> CSL;                    // this block's K blocks: rank, rank + cs, ... (one at least)
   int4* part = reinterpret_cast<int4*>(ring + p.stages * stage_bytes);   // [source block][token quad][128]: four tokens
   const int squads = ((p.ntok >> 2) + cs - 1) >> CSL;               // token quad Q belongs to block Q mod cs
   const uint32_t tmem_cols = nb <= 32 ? 32u : (nb <= 64 ? 64u : 128u);
@@ -179,6 +179,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) w8a8_gemv_tc_kernel(const __gri
   const uint32_t tmem = tmem_slot;
   const int row0 = tile * (p.dual ? 64 : 128);
 
+  int issued = 0;                          // the producer's K blocks so far
   if (warp == 0) {
     if (lane == 0) {
       const CUtensorMap* mw = &maps.w;
@@ -202,7 +203,8 @@ __global__ void __launch_bounds__(kTcThreads, 2) w8a8_gemv_tc_kernel(const __gri
       for (int i = 0; i < pre; ++i) weights(i, i);
       if (p.g.prefetch) grid_dependency_wait();
       for (int i = 0; i < pre; ++i) tokens(i, i);
-      int issued = pre, s = 0;
+      int s = 0;
+      issued = pre;
       for (int i = pre; i < nk; ++i) {
         if (abort_flag || !mbar_wait_bounded(&empty_bar[s], ((i / p.stages) & 1) ^ 1)) {
           report_status(p.g.status_word, LSVD_ERR_TIMEOUT);
@@ -214,8 +216,6 @@ __global__ void __launch_bounds__(kTcThreads, 2) w8a8_gemv_tc_kernel(const __gri
         ++issued;
         if (++s == p.stages) s = 0;
       }
-      if (abort_flag)                        // this block's copies must have landed before it may leave
-        for (int i = max(0, issued - p.stages); i < issued; ++i) mbar_wait_bounded(&full_bar[i % p.stages], (i / p.stages) & 1);
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -276,10 +276,6 @@ __global__ void __launch_bounds__(kTcThreads, 2) w8a8_gemv_tc_kernel(const __gri
       uint32_t v[16];
       __syncwarp();
       tmem_ld16(taddr + c, v);
-      if (nk == 0) {
-#pragma unroll
-        for (int e = 0; e < 16; ++e) v[e] = 0u;
-      }
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         if (c + 4 * q < p.g.m) {
@@ -300,11 +296,20 @@ __global__ void __launch_bounds__(kTcThreads, 2) w8a8_gemv_tc_kernel(const __gri
   } else {
     __syncthreads();
   }
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(tmem, tmem_cols);
+  if (warp < 2) {
+    // Whoever gave up, and whenever: the barrier above has ended every role, so the flag is final.  This block's copies must
+    // have landed before its shared memory goes, its MMAs have ended before their accumulators are released.
+    if (lane == 0 && abort_flag) {
+      if (warp == 1) mbar_wait_bounded(&acc_bar, 0);
+      else for (int i = max(0, issued - p.stages); i < issued; ++i) mbar_wait_bounded(&full_bar[i % p.stages], (i / p.stages) & 1);
+    }
+    __syncwarp();
+    if (warp == 1) {
+      tc_fence_after();
+      tmem_dealloc(tmem, tmem_cols);
+    }
+    return;
   }
-  if (warp < 2) return;
 
   if (!p.dual) {
     tc_epilogue<CSL, false, false>(p.g, part, sa, sb, w0, w1, squads, rank, row0, ew, lane);
@@ -316,7 +321,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) w8a8_gemv_tc_kernel(const __gri
 }
 
 // Blocks per tile: the cluster grows (to at most 8, the portable size) until the tiles fill the SMs once, as long as every
-// block keeps two K blocks.  45 MB gate/up pair at 32 tokens, 5504 channels (86 tiles): 2 blocks per tile 16.1 us with its
+// block keeps a K block.  45 MB gate/up pair at 32 tokens, 5504 channels (86 tiles): 2 blocks per tile 16.1 us with its
 // quantiser, 4 blocks 17.6; 45 MB down projection (32 tiles): 8 blocks 19.3, 4 blocks 21.
 // Shared memory: two blocks per SM (110 KB each), so that the blocks of the next product of a chain find room for their
 // first stages while this one drains; 76 KB measured 10 % slower on the mixffn step (fewer bytes in flight), 160 KB -- one
