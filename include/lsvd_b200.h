@@ -365,7 +365,9 @@ typedef struct lsvd_gemv_args {
                                  /* 1: persistent TMA-fed kernel with K split over warps, m <= 16 only   */
                                  /*    (LSVD_ERR_UNSUPPORTED beyond); 2: TMA-fed kernel whose warps      */
                                  /*    share the token rows (built for 17..64 tokens, valid for any m);   */
-                                 /* 3: register-fed kernel for any m; 4: tcgen05 kernel for any m.       */
+                                 /* 3: register-fed kernel for any m; 4: tcgen05 kernel for any m        */
+                                 /*    (LSVD_ERR_UNSUPPORTED for rows that overlap or lie 2^40 bytes     */
+                                 /*    apart; form 0 and 3 take any stride that is a multiple of 16).    */
                                  /* Same values in every form.                                           */
   uint32_t* row_absmax;          /* optional device words [m * row_absmax_stride]: see above (not forms 1, 2) */
   int64_t row_absmax_stride;     /* words between two tokens                                              */

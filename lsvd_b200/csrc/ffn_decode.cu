@@ -997,7 +997,13 @@ extern "C" int lsvd_w8a8_gemv(const lsvd_gemv_args* a, void* stream) {
   if (a->form == 1) return a->m <= 16 ? launch_gemv_streamed(p, dual, split, st) : LSVD_ERR_UNSUPPORTED;
   if (a->form == 2) return launch_gemv_wide(p, dual, split, st);
   if (a->form < 0 || a->form > 4) return LSVD_ERR_INVALID_ARG;
-  if (a->form == 4 || (a->form == 0 && tc_is_faster(a, dual))) return launch_gemv_tc(p, dual, split, st);
+  // What a tensor map describes: rows that do not overlap, less than 2^40 bytes apart.  Broadcast or overlapping rows, and the
+  // stride of a single row, are anything: plain loads take them.
+  auto mappable = [&](int rows, int64_t stride) { return rows == 1 || (stride >= a->k && stride < (1ll << 40)); };
+  const bool tma_ok = mappable(a->n, a->w_row_stride) && (!dual || mappable(a->n, a->w2_row_stride)) && mappable(a->m, a->a_row_stride) &&
+                      (!split || mappable(a->m, a->a2_row_stride));
+  if (a->form == 4 && !tma_ok) return LSVD_ERR_UNSUPPORTED;
+  if (a->form == 4 || (a->form == 0 && tma_ok && tc_is_faster(a, dual))) return launch_gemv_tc(p, dual, split, st);
   if (a->m <= 8) return launch_gemv_nt<1>(p, dual, split, st);
   if (a->m <= 16) return launch_gemv_nt<2>(p, dual, split, st);
   if (a->m <= 32) return launch_gemv_nt<4>(p, dual, split, st);

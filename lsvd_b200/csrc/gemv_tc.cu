@@ -336,8 +336,8 @@ int launch_gemv_tc(const GemvParams& g, bool dual, bool split, cudaStream_t st) 
   p.kb = (g.k + 127) / 128;
   int rc = make_map_k128(&maps.w, g.w, g.n, g.k, g.w_row_stride, 64);
   if (rc == LSVD_OK && dual) rc = make_map_k128(&maps.w2, g.w2, g.n, g.k, g.w2_row_stride, 64);
-  if (rc == LSVD_OK) rc = make_map_k128(&maps.a, g.a, g.m, g.k, g.a_row_stride, p.ntok);
-  if (rc == LSVD_OK && split) rc = make_map_k128(&maps.a2, g.a2, g.m, g.k, g.a2_row_stride, p.ntok);
+  if (rc == LSVD_OK) rc = make_map_k128(&maps.a, g.a, g.m, g.k, g.m == 1 ? g.k : g.a_row_stride, p.ntok);
+  if (rc == LSVD_OK && split) rc = make_map_k128(&maps.a2, g.a2, g.m, g.k, g.m == 1 ? g.k : g.a2_row_stride, p.ntok);
   if (rc != LSVD_OK) return rc;
   const int per = dual ? 64 : 128, tiles = (g.n + per - 1) / per;
   const int sms = std::max(1, device_sm_count());

@@ -72,3 +72,20 @@ def test_the_form_chosen_by_size_has_the_same_bits(m, n, k, dual):
         got = w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], want_acc=True, prefetch_weights=early, **kw)
         for x, y in zip(got, want):
             assert x is y is None or torch.equal(x, y)
+
+
+@pytest.mark.parametrize("early", [False, True])
+@pytest.mark.parametrize("m,n,k", [(1, 256, 8192), (5, 64, 512), (29, 64, 8192), (64, 1024, 4096)])
+def test_broadcast_and_overlapping_rows(m, n, k, early):
+    """Rows that no tensor map describes -- one activation row for all tokens, windows of one buffer as weights, any stride of a
+    single row -- give what their contiguous copies give, also where the size alone would choose the tcgen05 kernel."""
+    from lsvd_b200.ffn import w8a8_gemv
+    d = _case(m, n, k, False, False, seed=k)
+    one = d["a"][:1].contiguous().expand(m, k) if m > 1 else d["a"].contiguous().as_strided((1, k), (16, 1))
+    windows = torch.randint(-128, 128, (16 * n + k,), dtype=torch.int8, device="cuda").as_strided((n, k), (16, 1))
+    for a, w in ((one, d["w"]), (d["a"], windows), (one, windows)):
+        got = w8a8_gemv(a, d["sa"], w, d["ws"], want_acc=True, prefetch_weights=early)
+        want = w8a8_gemv(a.contiguous(), d["sa"], w.contiguous(), d["ws"], want_acc=True, form=3)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    with pytest.raises(ValueError):
+        w8a8_gemv(d["a"], d["sa"], windows, d["ws"], form=4)
