@@ -373,11 +373,13 @@ typedef struct lsvd_gemv_args {
   int64_t row_absmax_stride;     /* words between two tokens                                              */
   int32_t absmax_split;          /* 0: one word per token; else channels >= absmax_split (a multiple of  */
                                  /* 16) go to the token's second word                                     */
-  int32_t prefetch_weights;      /* every block asks for its weights (form 4: the first stages of its ring, form 3: */
-                                 /* L2 prefetch) before it waits for the kernel launched before it on the stream.    */
-                                 /* Set it only behind one of this library's kernels: the weights must be complete   */
-                                 /* when that kernel starts.  Form 0 then is the tcgen05 kernel.  Results do not     */
-                                 /* depend on it.                                                                    */
+  int32_t prefetch_weights;      /* 1: a hint, wherever the call stands: form 3 asks for its weight rows (L2        */
+                                 /*    prefetch) before it waits for the kernel in front of it on the stream.        */
+                                 /* 2: the tcgen05 kernel READS its first weights before that wait, and form 0 is    */
+                                 /*    that kernel.  Only directly behind a kernel that does not write weights and   */
+                                 /*    releases its dependents after its own wait (this library's quantisers) or     */
+                                 /*    behind a product launched so: everything that wrote the weights on the stream */
+                                 /*    must stand before that kernel.  Other forms take 2 as 1.                      */
   float* out_f32;                /* optional device fp32 [m, n] (single product, not forms 1 and 2): (acc * a_scale) * w_scale */
                                  /* with no fp16 rounding -- the partial sum a row-parallel rank sends to the all-reduce  */
 } lsvd_gemv_args;

@@ -242,7 +242,7 @@ extern "C" int lsvd_ffn_decode(const lsvd_ffn_decode_args* a, void* stream) {
 
   // 2. RTN gate/up pair: needs only x_q, runs beside the SVD branch
   lsvd_gemv_args gw{};
-  gw.prefetch_weights = 1;
+  gw.prefetch_weights = 2;
   gw.m = m; gw.n = n_q; gw.k = a->d_in;
   gw.w = a->Wg_q; gw.w_row_stride = a->d_in; gw.w_scale = a->Wg_s;
   gw.w2 = a->Wu_q; gw.w2_row_stride = a->d_in; gw.w2_scale = a->Wu_s;
@@ -260,7 +260,7 @@ extern "C" int lsvd_ffn_decode(const lsvd_ffn_decode_args* a, void* stream) {
 
   // 3. SVD branch: latents, their quantisation, gate/up from the latents
   lsvd_gemv_args gu{};
-  gu.prefetch_weights = 1;
+  gu.prefetch_weights = 2;
   gu.m = m; gu.n = 2 * r; gu.k = a->d_in;
   gu.w = a->U_q; gu.w_row_stride = a->d_in; gu.w_scale = a->U_s;
   gu.a = x_q; gu.a_row_stride = a->d_in; gu.a_scale = x_s; gu.a_scale_stride = 1;
@@ -270,7 +270,7 @@ extern "C" int lsvd_ffn_decode(const lsvd_ffn_decode_args* a, void* stream) {
   q1.rows = 2 * m; q1.cols = r; q1.x = lat16; q1.x_row_stride = r; q1.q = z_q; q1.q_row_stride = r; q1.scale = z_s;
   LSVD_TRY(lsvd_act_quant(&q1, st));
   lsvd_gemv_args gv{};
-  gv.prefetch_weights = 1;
+  gv.prefetch_weights = 2;
   gv.m = m; gv.n = a->n_svd; gv.k = r;
   gv.w = a->Vg_q; gv.w_row_stride = r; gv.w_scale = a->Vg_s;
   gv.w2 = a->Vu_q; gv.w2_row_stride = r; gv.w2_scale = a->Vu_s;
@@ -299,7 +299,7 @@ extern "C" int lsvd_ffn_decode(const lsvd_ffn_decode_args* a, void* stream) {
 
   // 5. down projection (+ residual)
   lsvd_gemv_args gd{};
-  gd.prefetch_weights = 1;
+  gd.prefetch_weights = 2;
   gd.m = m; gd.n = a->d_out; gd.k = a->d_ffn;
   gd.w = a->Wd_q; gd.w_row_stride = a->d_ffn; gd.w_scale = a->Wd_s;
   gd.a = h_q; gd.a_row_stride = a->d_ffn; gd.a_scale = h_s; gd.a_scale_stride = 1;

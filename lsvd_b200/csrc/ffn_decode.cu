@@ -952,7 +952,7 @@ namespace lsvd {
 //   64 tokens: 1024 x 512 10.3 / 10.3, 4096 x 512 10.3 / 11.4, 1024 x 1024 pair 18.4 / 14.4, 5504 x 512 pair 20.5 / 16.4;
 //              4 MB and more 16.4 / 12.4 to 75.9 / 41.0 (the shared-token form, which took these before).
 static bool tc_is_faster(const lsvd_gemv_args* a, bool dual) {
-  if (a->prefetch_weights != 0) return true;
+  if (a->prefetch_weights == 2) return true;
   const int64_t bytes = static_cast<int64_t>(a->n) * a->k * (dual ? 2 : 1);
   if (a->k >= 8192) return true;
   if (!dual && a->n >= 16384 && (a->m > 16 || (a->m > 8 && a->k >= 256))) return true;
@@ -990,7 +990,7 @@ extern "C" int lsvd_w8a8_gemv(const lsvd_gemv_args* a, void* stream) {
   p.m = a->m; p.n = a->n; p.k = a->k; p.epilogue = a->epilogue;
   p.row_absmax = a->row_absmax; p.row_absmax_stride = a->row_absmax_stride;
   p.absmax_split = a->absmax_split > 0 ? a->absmax_split : a->n;
-  p.prefetch = (a->prefetch_weights != 0 && ffn_chain_enabled()) ? 1 : 0;
+  p.prefetch = ffn_chain_enabled() ? a->prefetch_weights : 0;
   p.out_f32 = a->out_f32;
   if (a->out_f32 != nullptr && (dual || a->form == 1 || a->form == 2)) return LSVD_ERR_UNSUPPORTED;
   cudaStream_t st = static_cast<cudaStream_t>(stream);

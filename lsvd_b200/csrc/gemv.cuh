@@ -18,7 +18,8 @@ struct GemvParams {
   // optional per-token maximum of |fp32 value| over the output channels, kept as the bit pattern of a non-negative
   // float (ordered like an unsigned integer): slot 0 for channels below absmax_split, slot 1 from there on
   uint32_t* row_absmax; int64_t row_absmax_stride; int32_t absmax_split;
-  int32_t prefetch;          // request weights before waiting for the previous kernel (launched programmatically)
+  int32_t prefetch;          // before the wait for the previous kernel (launched programmatically): 1 weights toward L2 (register-fed
+                             // form only), 2 weights read (tcgen05 form)
   float* out_f32;            // optional [m, n]: (acc * a_scale) * w_scale before any fp16 rounding (single products)
 };
 

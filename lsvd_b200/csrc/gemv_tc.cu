@@ -10,7 +10,7 @@
 //     its K range block by block (block r of c takes the 128-byte K blocks r, r + c, ..., so that the cluster reads
 //     adjacent bytes of a row at the same time); their exact int32 sums meet in distributed shared memory, token quad q in
 //     block q mod c, which adds them and runs the epilogue for its tokens.
-//   * With `prefetch` the first stages' weights are requested before griddepcontrol.wait: they travel while the quantiser in front of the
+//   * With prefetch 2 the first stages' weights are requested before griddepcontrol.wait: they travel while the quantiser in front of the
 //     product is still running (programmatic stream serialisation), which takes the ramp-up of the stream out of the
 //     chain of short dependent kernels that a decode step is.
 // Measured against the mma.sync forms it replaced as the default (B200, graph replay of quantiser + product, weights
@@ -330,6 +330,7 @@ int launch_gemv_tc(const GemvParams& g, bool dual, bool split, cudaStream_t st) 
   TcMaps maps;
   TcParams p{};
   p.g = g;
+  p.g.prefetch = g.prefetch == 2 ? 1 : 0;          // a hint does not say that the weights are complete
   p.dual = dual ? 1 : 0;
   p.split = split ? 1 : 0;
   p.ntok = (g.m + 15) / 16 * 16;
@@ -350,7 +351,7 @@ int launch_gemv_tc(const GemvParams& g, bool dual, bool split, cudaStream_t st) 
   void (*kern)(TcMaps, TcParams) = csl == 0 ? w8a8_gemv_tc_kernel<0> : csl == 1 ? w8a8_gemv_tc_kernel<1>
                                    : csl == 2 ? w8a8_gemv_tc_kernel<2> : w8a8_gemv_tc_kernel<3>;
   LSVD_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
-  LSVD_CUDA_TRY(launch_chained(kern, dim3(tiles << csl), dim3(kTcThreads), smem, st, 1 << csl, g.prefetch != 0, maps, p));
+  LSVD_CUDA_TRY(launch_chained(kern, dim3(tiles << csl), dim3(kTcThreads), smem, st, 1 << csl, p.g.prefetch != 0, maps, p));
   return LSVD_OK;
 }
 

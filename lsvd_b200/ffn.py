@@ -175,7 +175,9 @@ def w8a8_gemv(a_q, a_scale, w_q, w_scale, w2_q=None, w2_scale=None, a2_q=None, a
     ``form`` 0 is chosen by size, 1 the persistent TMA-fed kernel (at most 16 tokens), 2 the wide one, 3 the
     register-fed one, 4 the tcgen05 one; ``status_word`` (int32 device tensor) receives LSVD_ERR_TIMEOUT if a pipeline wait gives up.  ``fp32_swiglu`` selects the
     all-fp32 gate/up epilogue ``up * (gate * sigmoid(gate))``; ``row_absmax`` (int32 view of the words, strided by
-    token) collects max |fp32 value| per token, channels from ``absmax_split`` on in the token's second word."""
+    token) collects max |fp32 value| per token, channels from ``absmax_split`` on in the token's second word.
+    ``prefetch_weights`` True is a hint that is safe anywhere; 2 lets the kernel read weights before it waits for the launch in
+    front of it, which must be one of this library's quantisers (or a product launched so) with the weights complete before it."""
     _require_cuda(a_q, w_q)
     m, k = a_q.shape
     n = w_q.shape[0]
@@ -206,7 +208,7 @@ def w8a8_gemv(a_q, a_scale, w_q, w_scale, w2_q=None, w2_scale=None, a2_q=None, a
     if residual is not None:
         g.residual, g.residual_row_stride = residual.data_ptr(), residual.stride(0)
     g.form, g.status_word = form, _ptr(status_word)
-    g.prefetch_weights = 1 if prefetch_weights else 0
+    g.prefetch_weights = int(prefetch_weights)
     _lib.check(_lib.load().lsvd_w8a8_gemv(C.byref(g), _stream_ptr(a_q)))
     return out, acc, acc2
 

@@ -51,7 +51,7 @@ class LSVDDecoderLayer(nn.Module):
         the place for the device-side move to the next token (``decode_advance``) of a decode loop."""
         lay, H, B = self.layout, self.layout.num_heads, x.shape[0]
         xq, xs, xn = act_quant(x, want_rotated=True, norm_weight=self.ln1, norm_eps=1e-5)
-        lat, _, _ = w8a8_gemv(xq, xs, self.W_lat_q, self.W_lat_s, prefetch_weights=True)
+        lat, _, _ = w8a8_gemv(xq, xs, self.W_lat_q, self.W_lat_s, prefetch_weights=2)
         lk = lat[:, self.Rq:self.Rq + lay.sum_k]
         lv = None if lay.shared_kv else lat[:, self.Rq + lay.sum_k:]       # shared: one latent per head serves K and V
         cache_append(lay, lk, lv, infer_state.mem_index, cache_k, scale_k, cache_v, scale_v)
@@ -72,7 +72,7 @@ class LSVDDecoderLayer(nn.Module):
             with torch.cuda.stream(side):
                 after_attention()
         oq, os_, _ = act_quant(o_lat)
-        y1, _, _ = w8a8_gemv(oq, os_, self.W_uvo_q, self.W_uvo_s, residual=xn, prefetch_weights=True)
+        y1, _, _ = w8a8_gemv(oq, os_, self.W_uvo_q, self.W_uvo_s, residual=xn, prefetch_weights=2)
         out = self.ffn(y1, out=out, norm_weight=self.ln2, norm_eps=1e-6, residual=y1)
         if side is not None:
             torch.cuda.current_stream(x.device).wait_stream(side)

@@ -53,7 +53,7 @@ def test_accumulators_and_results(m, n, k, kind):
         assert torch.equal(o32[0], o32[1])
     words = [torch.zeros(m, 4, dtype=torch.int32, device="cuda") for _ in range(2)]
     outs = [w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], fp32_swiglu=dual, row_absmax=words[i], absmax_split=16 if n > 16 else 0,
-                      form=4 - i, prefetch_weights=i == 0, **kw)[0] for i in range(2)]
+                      form=4 - i, prefetch_weights=2 * (i == 0), **kw)[0] for i in range(2)]
     assert torch.equal(outs[0], outs[1])
     assert torch.equal(words[0], words[1])
 
@@ -62,19 +62,19 @@ def test_accumulators_and_results(m, n, k, kind):
                                         (17, 16384, 16, False), (17, 8192, 4096, False), (16, 8192, 4096, False), (33, 1024, 4096, False), (33, 1008, 4096, False), (33, 1024, 1024, True),
                                         (33, 1008, 1024, True)])
 def test_the_form_chosen_by_size_has_the_same_bits(m, n, k, dual):
-    """Both sides of each line of the choice, with and without an early request for the weights."""
+    """Both sides of each line of the choice: without a hint, with one, and with the early read (nothing wrote the weights)."""
     from lsvd_b200.ffn import w8a8_gemv
     d = _case(m, n, k, dual, False, seed=n)
     kw = dict(w2_q=d["w2"], w2_scale=d["ws2"]) if dual else {}
     want = w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], want_acc=True, form=3, **kw)
     torch.cuda.synchronize()
-    for early in (False, True):
+    for early in (False, True, 2):
         got = w8a8_gemv(d["a"], d["sa"], d["w"], d["ws"], want_acc=True, prefetch_weights=early, **kw)
         for x, y in zip(got, want):
             assert x is y is None or torch.equal(x, y)
 
 
-@pytest.mark.parametrize("early", [False, True])
+@pytest.mark.parametrize("early", [False, 2])
 @pytest.mark.parametrize("m,n,k", [(1, 256, 8192), (5, 64, 512), (29, 64, 8192), (64, 1024, 4096)])
 def test_broadcast_and_overlapping_rows(m, n, k, early):
     """Rows that no tensor map describes -- one activation row for all tokens, windows of one buffer as weights, any stride of a
@@ -89,3 +89,61 @@ def test_broadcast_and_overlapping_rows(m, n, k, early):
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     with pytest.raises(ValueError):
         w8a8_gemv(d["a"], d["sa"], windows, d["ws"], form=4)
+
+
+@pytest.mark.parametrize("form", [0, 3, 4])
+def test_hint_behind_the_kernel_that_writes_the_weights(form):
+    """``prefetch_weights=True`` is a hint wherever the call stands, directly behind a copy into the weights too."""
+    from lsvd_b200.ffn import w8a8_gemv
+    d = _case(8, 4096, 8192, False, False, seed=3)
+    other = _case(8, 4096, 8192, False, False, seed=4)["w"]
+    want = [w8a8_gemv(d["a"], d["sa"], w.clone(), d["ws"], form=3)[0] for w in (d["w"], other)]
+    w = d["w"].clone()
+    got = []
+    for i in range(20):
+        w.copy_(other if i % 2 else d["w"])
+        got.append(w8a8_gemv(d["a"], d["sa"], w, d["ws"], form=form, prefetch_weights=True)[0])
+    assert all(torch.equal(y, want[i % 2]) for i, y in enumerate(got))
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_weights_rewritten_on_the_stream_right_before_a_step(graph):
+    """A step whose products read weights before their wait sees what was written to them in front of its first quantiser: the
+    hybrid FFN (both streams) and the mixffn structure, eager and captured with the copies."""
+    from lsvd_b200 import synth
+    from lsvd_b200.ffn import HybridFFN
+    from lsvd_b200.mixffn import MixedFFNGateUpDenseLatentFused
+    from oracle import mixffn as omix
+    hk = synth.sign_matrix(12, seed=0).float()
+    cuda = lambda w: {k: v.cuda() if isinstance(v, torch.Tensor) else v for k, v in w.items()}
+    gen = torch.Generator().manual_seed(4)
+    mk = lambda o, i: (torch.randn(o, i, generator=gen) / i ** 0.5).half()
+    mix = lambda: omix.convert_swiglu(mk(1024, 512), mk(1024, 512), mk(512, 1024), torch.randn(512, generator=gen).half(), 0.5, 0.5, 64, gen)
+    for make, ws in ((HybridFFN, [synth.ffn_weights(1024, 12 * 64, 128, 384, seed=s, had_K=hk, K=12) for s in (1, 2)]),
+                     (MixedFFNGateUpDenseLatentFused, [mix(), mix()])):
+        mods = [make(cuda(w)) for w in ws]
+        live = make(cuda(ws[0]))
+        x = torch.randn(5, 1024 if make is HybridFFN else 512, generator=gen).half().cuda()
+        want = [m(x).clone() for m in mods]
+        assert not torch.equal(*want)
+
+        def step(i):
+            for mine, given in zip(live.buffers(), mods[i].buffers()):
+                mine.copy_(given)
+            return live(x)
+        if graph:
+            step(0)
+            torch.cuda.synchronize()
+            graphs = []
+            for i in range(2):
+                g = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(g):
+                    y = step(i)
+                graphs.append((g, y))
+            for _ in range(10):
+                for i, (g, y) in enumerate(graphs):
+                    g.replay()
+                    assert torch.equal(y, want[i])
+        else:
+            got = [step(i % 2).clone() for i in range(20)]
+            assert all(torch.equal(y, want[i % 2]) for i, y in enumerate(got))
