@@ -37,8 +37,8 @@ cudaError_t ensure_large_l1(const void* kernel);
 // with programmatic stream serialisation: the next kernel's blocks may become resident while the previous
 // kernel drains, and wait in grid_dependency_sync() (first statement of every such kernel) until the previous
 // grid has completed and its writes are visible.  LSVD_CHAINED_LAUNCH=0 in the environment turns it off.
-// The attention kernels, the quantisers and the products that ask for a weight prefetch use it (LSVD_CHAIN_FFN=0 turns
-// the products' prefetch off).
+// The attention kernels, the quantisers and the products that ask for a weight prefetch use it (LSVD_CHAIN_FFN=0 launches
+// the quantisers and the products plainly, and no product asks for weights early).
 bool chained_launch_enabled();
 bool ffn_chain_enabled();
 

@@ -743,7 +743,7 @@ extern "C" int lsvd_act_quant(const lsvd_act_quant_args* a, void* stream) {
   if (rotate && a->cols == 4096 && p.vec8 && p.norm_weight == nullptr && p.fake == nullptr && aligned(a->q, 16) && (a->q_row_stride % 16) == 0 &&
       (p.x_rot == nullptr || aligned(p.x_rot, 16))) {
     LSVD_CUDA_TRY(launch_chained(act_quant_rot4096_kernel, dim3(a->rows), dim3(256), 0, static_cast<cudaStream_t>(stream), 1,
-                                 true, p));
+                                 ffn_chain_enabled(), p));
     return LSVD_OK;
   }
   // many rows of a width the warp-per-row kernel is built for (a prefill): no shared memory, no block barriers
@@ -761,7 +761,7 @@ extern "C" int lsvd_act_quant(const lsvd_act_quant_args* a, void* stream) {
       default: break;
     }
     if (kern != nullptr) {
-      LSVD_CUDA_TRY(launch_chained(kern, dim3((a->rows + 7) / 8), dim3(256), 0, static_cast<cudaStream_t>(stream), 1, true, p));
+      LSVD_CUDA_TRY(launch_chained(kern, dim3((a->rows + 7) / 8), dim3(256), 0, static_cast<cudaStream_t>(stream), 1, ffn_chain_enabled(), p));
       return LSVD_OK;
     }
   }
@@ -771,12 +771,12 @@ extern "C" int lsvd_act_quant(const lsvd_act_quant_args* a, void* stream) {
     const int chunks = a->cols / 8;
     const int threads = std::min(1024, (chunks + 31) / 32 * 32);
     LSVD_CUDA_TRY(launch_chained(chunks <= 1024 ? act_quant_block_kernel<1> : act_quant_block_kernel<2>, dim3(a->rows), dim3(threads), 0,
-                                 static_cast<cudaStream_t>(stream), 1, true, p));
+                                 static_cast<cudaStream_t>(stream), 1, ffn_chain_enabled(), p));
     return LSVD_OK;
   }
   const int smem = a->cols * 4;
   if (smem > 48 * 1024) LSVD_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(act_quant_kernel), smem));
-  LSVD_CUDA_TRY(launch_chained(act_quant_kernel, dim3(a->rows), dim3(256), smem, static_cast<cudaStream_t>(stream), 1, true, p));
+  LSVD_CUDA_TRY(launch_chained(act_quant_kernel, dim3(a->rows), dim3(256), smem, static_cast<cudaStream_t>(stream), 1, ffn_chain_enabled(), p));
   return LSVD_OK;
 }
 
@@ -812,7 +812,7 @@ extern "C" int lsvd_heads_hadamard_quant(const lsvd_heads_hadamard_quant_args* a
     return LSVD_OK;
   }
   if (kern == nullptr) return LSVD_ERR_UNSUPPORTED;       // not a power of two and no had_K given
-  LSVD_CUDA_TRY(launch_chained(kern, dim3(a->rows), dim3(128), 0, static_cast<cudaStream_t>(stream), 1, true, p));
+  LSVD_CUDA_TRY(launch_chained(kern, dim3(a->rows), dim3(128), 0, static_cast<cudaStream_t>(stream), 1, ffn_chain_enabled(), p));
   return LSVD_OK;
 }
 
@@ -936,7 +936,7 @@ extern "C" int lsvd_hadamard_quant(const lsvd_hadamard_quant_args* a, void* stre
   // calls 48.1 us plain / 50.2 chained at 297 tokens, 51.2 / 52.8 at 500, but 26.8 / 26.4 at 148; 20 x 8 9.4 / 9.1 at 500.
   const bool chain = smem <= 16 * 1024 || a->rows <= 2 * device_sm_count();
   LSVD_CUDA_TRY(launch_chained(kern, dim3(static_cast<unsigned>(a->rows * p.cluster)), dim3(256), smem,
-                               static_cast<cudaStream_t>(stream), p.cluster, chain, p));
+                               static_cast<cudaStream_t>(stream), p.cluster, chain && ffn_chain_enabled(), p));
   return LSVD_OK;
 }
 

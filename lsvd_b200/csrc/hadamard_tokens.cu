@@ -191,7 +191,7 @@ static int launch_tokens(const HadQuantParams& p, cudaStream_t st) {
   const int sms = std::max(1, device_sm_count());
   void (*kern)(HadQuantParams) = hadamard_tokens_kernel<KT, NB, PER_SM>;
   if (smem > 48 * 1024) LSVD_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
-  LSVD_CUDA_TRY(launch_chained(kern, dim3(std::min(p.rows, PER_SM * sms)), dim3(KT * 32), smem, st, 1, true, p));
+  LSVD_CUDA_TRY(launch_chained(kern, dim3(std::min(p.rows, PER_SM * sms)), dim3(KT * 32), smem, st, 1, ffn_chain_enabled(), p));
   return LSVD_OK;
 }
 

@@ -347,3 +347,43 @@ def test_provider_converts_a_swiglu_module_and_matches_the_oracle():
     ref = offn.hybrid_ffn_stages(xn, w)["out"]
     ref = (ref.float() + x2.float()).half()
     assert rel_to_norm(y.reshape(-1, hidden).cpu().float(), ref.float()) < TOL
+
+
+@pytest.mark.parametrize("chain", ["0", "1"])
+def test_switch_for_plain_launches_covers_the_quantisers(chain):
+    """LSVD_CHAIN_FFN=0: no launch of the FFN step depends programmatically on the one in front of it (edges of the captured
+    graph), and the results are those of the default."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch
+from cuda.bindings import runtime as rt
+from lsvd_b200 import synth
+from lsvd_b200.ffn import HybridFFN
+w = synth.ffn_weights(1024, 12 * 64, 128, 384, seed=1, had_K=synth.sign_matrix(12, seed=0).float(), K=12)
+ffn = HybridFFN({k: v.cuda() if isinstance(v, torch.Tensor) else v for k, v in w.items()})
+x = torch.randn(5, 1024, generator=torch.Generator().manual_seed(1)).half().cuda()
+ffn(x)
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph(keep_graph=True)
+with torch.cuda.graph(g):
+    y = ffn(x)
+g.instantiate()
+g.replay()
+raw = rt.cudaGraph_t(g.raw_cuda_graph())
+n = rt.cudaGraphGetEdges_v2(raw)[-1]
+err, _, _, data, _ = rt.cudaGraphGetEdges_v2(raw, n)
+assert err == rt.cudaError_t.cudaSuccess
+prog = rt.cudaGraphDependencyType.cudaGraphDependencyTypeProgrammatic
+print("EDGES", n, sum(int(d.type) == int(prog) for d in data), y.double().abs().sum().item())
+"""
+    out = []
+    for env in (chain, "1"):
+        r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, LSVD_CHAIN_FFN=env), capture_output=True, text=True, timeout=300,
+                           cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+        assert r.returncode == 0, r.stderr[-2000:]
+        out.append(next(l for l in r.stdout.splitlines() if l.startswith("EDGES")).split())
+    edges, programmatic = int(out[0][1]), int(out[0][2])
+    assert edges >= 6 and (programmatic == 0 if chain == "0" else programmatic >= 4)
+    assert out[0][3] == out[1][3]
