@@ -1,8 +1,8 @@
 // Hybrid SVD/RTN FFN for decode batches (1..64 tokens): per-token int8 quantisation (with the input and
 // the d_ffn Hadamard rotations), and the weight-streaming W8A8 products.
 //
-// The products are HBM streams of int8 weights: 100 MB per FFN call at the 7B shape whatever the batch.
-// A block owns 16 output channels (of one matrix, or of a gate/up pair); its eight warps split K, each
+// The products are HBM streams of int8 weights: 100 MB per FFN call at the 7B shape whatever the batch.  The FFN's chains run
+// the tcgen05 form (gemv_tc.cu); in the register-fed form here a block owns 16 output channels (of one matrix, or of a gate/up pair); its eight warps split K, each
 // lane loads 16 contiguous weight bytes per instruction straight into the A fragments of exact int8
 // tensor-core MMAs (m16n8k32, int32 accumulators) whose B fragments are the tokens' int8 activations
 // (L1/L2 resident), and the warps' partial sums meet in shared memory for the dequantising epilogue.

@@ -423,7 +423,7 @@ __device__ __forceinline__ void latent_quant_unit(const FusedParams& p, const FO
 }
 
 // (H_K kron H_64) rotation + per-token quantisation, one (token, group of 8 columns) unit per block: the arithmetic
-// of hadamard_quant_rows_kernel (ffn_decode.cu).  Every unit rotates all K blocks of 64 entries (cheap) and keeps the
+// of hadamard_tokens_kernel (hadamard_tokens.cu).  Every unit rotates all K blocks of 64 entries (cheap) and keeps the
 // 8 columns it owns, multiplies them by had_K on the tensor cores (the fragments of had_K are requested before
 // anything else, so that their latency hides behind the rotation), and the 8 units of a token agree on the row's
 // absmax through one atomic maximum and a counter they alone wait on (bounded), then quantise from registers.

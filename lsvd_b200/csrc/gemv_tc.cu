@@ -13,10 +13,10 @@
 //   * With prefetch 2 the first stages' weights are requested before griddepcontrol.wait: they travel while the quantiser in front of the
 //     product is still running (programmatic stream serialisation), which takes the ramp-up of the stream out of the
 //     chain of short dependent kernels that a decode step is.
-// Measured against the mma.sync forms it replaced as the default (B200, graph replay of quantiser + product, weights
-// from HBM): the stream itself runs at 6 TB/s; a block spends about 1 us on its start and 1.5 to 3 us on the sums and the
-// epilogue.  Hybrid FFN 4096/11008 at 1 / 29 tokens 51.3 / 62.2 -> 45.3 / 55.5 us per call, 5120/13824 at 64 tokens
-// 159 -> 88 us, mixffn 4096/14336 at 32 tokens 124 -> 79 us.
+// Measured against the mma.sync forms in the FFN's chains (B200, graph replay): hybrid FFN 4096/11008 at 1 / 29 tokens
+// 51.3 / 62.2 -> 45.3 / 55.5 us per call, 5120/13824 at 64 tokens 159 -> 88 us, mixffn 4096/14336 at 32 tokens 124 -> 79 us.
+// A launch on its own (ncu, cold) is bound by its start, the sums and the epilogue: 45 MB pair 19.8 us, 45 MB down projection
+// 15.3, 4 MB 7.8 at 16 tokens; 58.7 MB pair 19.0 at 32 (3.1 TB/s).  A block's start takes about 1 us, sums and epilogue 1.5 to 3.
 // Every wait on an mbarrier is bounded; one that gives up, in whatever role, reports LSVD_ERR_TIMEOUT, and the block still
 // attends the cluster barriers, waits for its own copies and MMAs and releases its tensor memory.
 #include <algorithm>
