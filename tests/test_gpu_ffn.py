@@ -132,7 +132,7 @@ def test_gemv_shapes_dual_and_down(m, n, k, split):
                                         (16, 5504, 4096, "dual"), (9, 688, 4096, "dual"), (16, 5504, 512, "split"),
                                         (3, 64, 48, "split")])
 def test_gemv_tma_form_equals_register_form(m, n, k, kind):
-    """form 1 (persistent, TMA-fed, at most 16 tokens) against form 0 and the oracle: same integers, same fp16."""
+    """form 1 (persistent, TMA-fed, at most 16 tokens) against form 3 (register-fed) and the oracle: same integers, same fp16."""
     gen = torch.Generator().manual_seed(m * 11 + n + k)
     a = torch.randint(-128, 128, (m, k), generator=gen, dtype=torch.int8).cuda()
     w = torch.randint(-128, 128, (n, k), generator=gen, dtype=torch.int8).cuda()
@@ -146,7 +146,7 @@ def test_gemv_tma_form_equals_register_form(m, n, k, kind):
         kw["a2_q"] = torch.randint(-128, 128, (m, k), generator=gen, dtype=torch.int8).cuda()
         kw["a2_scale"] = (torch.rand(m, generator=gen) * 0.02 + 1e-3).cuda()
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
-    o0, acc0, acc0b = w8a8_gemv(a, sa, w, sw, want_acc=True, form=0, **kw)
+    o0, acc0, acc0b = w8a8_gemv(a, sa, w, sw, want_acc=True, form=3, **kw)
     o1, acc1, acc1b = w8a8_gemv(a, sa, w, sw, want_acc=True, form=1, status_word=status, **kw)
     assert int(status.item()) == 0
     assert torch.equal(acc1.cpu(), offn._i32_matmul(a.cpu(), w.cpu()))
@@ -298,7 +298,7 @@ def test_hadamard_across_heads_reference_fixture_and_7b_shape():
                                         (64, 1728, 5120, "dual"), (64, 3456, 5120, "dual"), (64, 1920, 5120, "single"),
                                         (64, 1280, 5120, "single"), (48, 2400, 2048 + 64, "split")])
 def test_gemv_wide_form_equals_register_form(m, n, k, kind):
-    """form 2 (token rows shared through shared memory, the default beyond 32 tokens) against form 3 (register-fed)
+    """form 2 (token rows shared through shared memory) against form 3 (register-fed)
     and the oracle: same integers, same fp16."""
     gen = torch.Generator().manual_seed(m * 13 + n + k)
     a = torch.randint(-128, 128, (m, k), generator=gen, dtype=torch.int8).cuda()

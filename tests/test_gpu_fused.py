@@ -1,5 +1,5 @@
 """The hybrid FFN as ONE persistent kernel (lsvd_ffn_decode with `fused`) against the chain of launches and the
-CPU oracle: the two forms run the same device functions, so every output must be bit-identical; the oracle bounds
+CPU oracle: the two forms run the same arithmetic in the same order, so every output must be bit-identical; the oracle bounds
 the end-to-end error (2e-3 * ||y_ref||_2, BASELINE tolerance for fp16 outputs).
 """
 import ctypes as C
