@@ -523,10 +523,6 @@ constexpr int kRingBytesPerWarp = 9088;              // two steps of a 64 + 64-r
 constexpr int kRingMaxStages = 4;
 
 __device__ __forceinline__ uint4 lds128(const uint8_t* p) { return *reinterpret_cast<const uint4*>(p); }
-// 16 bytes global -> shared without a register in between; a thread's copies complete in commit groups.
-__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 // Waits until at most `newer` of this thread's commit groups are still in flight (newer = 0..3).
 __device__ __forceinline__ void cp_async_wait_newer(int newer) {

@@ -158,6 +158,11 @@ __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, u
                : "memory");
 }
 
+// 16 bytes global -> shared without a register in between; a thread's copies complete in commit groups.
+__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
+}
+
 // Named barrier `id` of `count` threads that also ORs a flag over them: every participant gets the same answer, so a
 // decision to stop (a bounded wait that gave up somewhere) is taken by all of them or by none -- nobody is left
 // waiting alone at the next barrier.

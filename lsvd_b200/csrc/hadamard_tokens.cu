@@ -29,10 +29,6 @@ __device__ __forceinline__ void ldsm_x4_trans(uint32_t (&d)[4], uint32_t addr) {
                : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(addr) : "memory");
 }
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-
 template <int KT, int NB, int PER_SM>
 __global__ void __launch_bounds__(KT * 32, PER_SM) hadamard_tokens_kernel(const __grid_constant__ HadQuantParams p) {
   constexpr int kThreads = KT * 32;
