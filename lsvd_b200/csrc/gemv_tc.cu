@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) w8a8_gemv_tc_kernel(const __gri
   __shared__ uint64_t full_bar[kTcMaxStages], empty_bar[kTcMaxStages], acc_bar;
   __shared__ uint32_t tmem_slot;
   __shared__ volatile uint32_t abort_flag;
+  __shared__ int issued;                   // K blocks that the producer has requested (a register live to the end: 10 % a call)
   __shared__ float sa[64], sb[64];         // token scales of this block's token slots
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -169,6 +170,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) w8a8_gemv_tc_kernel(const __gri
     }
     mbar_init(&acc_bar, 1);
     abort_flag = 0;
+    issued = nk;
     fence_mbar_init();
   }
   if (warp == 1) tmem_alloc(&tmem_slot, tmem_cols);
@@ -179,7 +181,6 @@ __global__ void __launch_bounds__(kTcThreads, 2) w8a8_gemv_tc_kernel(const __gri
   const uint32_t tmem = tmem_slot;
   const int row0 = tile * (p.dual ? 64 : 128);
 
-  int issued = 0;                          // the producer's K blocks so far
   if (warp == 0) {
     if (lane == 0) {
       const CUtensorMap* mw = &maps.w;
@@ -204,16 +205,15 @@ __global__ void __launch_bounds__(kTcThreads, 2) w8a8_gemv_tc_kernel(const __gri
       if (p.g.prefetch) grid_dependency_wait();
       for (int i = 0; i < pre; ++i) tokens(i, i);
       int s = 0;
-      issued = pre;
       for (int i = pre; i < nk; ++i) {
         if (abort_flag || !mbar_wait_bounded(&empty_bar[s], ((i / p.stages) & 1) ^ 1)) {
           report_status(p.g.status_word, LSVD_ERR_TIMEOUT);
           abort_flag = 1;
+          issued = i;
           break;
         }
         weights(i, s);
         tokens(i, s);
-        ++issued;
         if (++s == p.stages) s = 0;
       }
     }
